@@ -673,7 +673,7 @@ static double h_min_norm(int ebit) { return ebit == 0 ? 0.0 : (ebit == 1 ? 1.0 :
 static double h_min_subnorm(int ebit, int mbit) { return ldexp(1.0, 2 - (1 << (ebit - 1)) - mbit); }
 
 // Micro-scale tables (src/quantizer.py:745-770), values as fp16 arithmetic produces them.
-static int l2_tables(int scheme, int bits, float tab[2][16])
+int l2_tables(int scheme, int bits, float tab[2][16])
 {
     const int n = 1 << bits;
     int ns = 1;
