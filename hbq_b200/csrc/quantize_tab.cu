@@ -25,11 +25,22 @@
 namespace hbq {
 
 constexpr int TAB_THREADS = 512;
+constexpr int MIX_THREADS = 384;            // 80 registers a thread at two CTAs per SM
 constexpr int TAB_SLOTS = 32;               // formats that can have a device table at the same time
 constexpr int TAB_MAX_ENTRIES = 8192;       // 32 KB per table
 
 // The staged tables.  In host code this name is only a handle for cudaGetSymbolAddress.
 static __device__ __align__(128) uint32_t g_tab_slots[TAB_SLOTS][TAB_MAX_ENTRIES];
+
+// The second candidate table of the two-table ("Mix") weight formats, as TabArgs describes the first.
+struct TabSecond {
+    const uint32_t* table;
+    int entries;
+    uint32_t base2, hi2, big_l1;
+    float inv_ele_max;
+    uint32_t nt2[4];
+    float tabf[4];
+};
 
 struct TabArgs {
     const uint4* x;
@@ -50,6 +61,7 @@ struct TabArgs {
     int log2Gt;               // log2(lanes per block)
     int m_lanes, log2m;       // chunks (= lanes) per micro-block
     int l2_sc_bit, nl2, l2_bytes;
+    TabSecond b;              // hbq_tab_mix_kernel
 };
 static_assert(sizeof(TabArgs) <= 4000, "kernel parameters are limited to 4 KB");
 
@@ -116,6 +128,32 @@ __device__ __forceinline__ int first_min4(const float* acc)
     return (int)(min(min(k0, k1), min(k2, k3)) & 3u);
 }
 
+// The eight element codes of a chunk: cw = its element values as fp16 pairs (non-negative), sg = words whose bits 15
+// and 31 are the elements' signs.  A value times 2^-14 is, as an fp16 pattern, the code shifted left by 10 - MB (the
+// code's exponent and mantissa fields ARE the pattern's low exponent bits and top mantissa bits, subnormal codes
+// included), so one multiply per pair replaces the field extraction (HBQ-A activations [8192, 8192] bf16 to packed
+// planes and the bf16 tensor: 113 -> 95 us).  E2M1: nibbles with the sign on top, E2M2:
+// magnitude nibbles and the signs in `sbits`.
+template <int MB>
+__device__ __forceinline__ uint32_t pack_codes(const uint32_t* cw, const uint32_t* sg, uint32_t& sbits)
+{
+    uint32_t v[4];
+    #pragma unroll
+    for (int p = 0; p < 4; ++p)
+        v[p] = h2_bits(__hmul2(bits_h2(cw[p]), bits_h2(0x04000400u))) | (sg[p] & 0x80008000u);
+    // the high bytes of the elements: {sign, -, -, -, code} (E2M2), {sign, -, -, -, code, -} (E2M1)
+    const uint32_t t0 = prmt(v[0], v[1], 0x7531u), t1 = prmt(v[2], v[3], 0x7531u);
+    const uint32_t ev = prmt(t0, t1, 0x6420u), od = prmt(t0, t1, 0x7531u);
+    if (MB == 1) {
+        const uint32_t e = ((ev >> 1) & 0x07070707u) | ((ev >> 4) & 0x08080808u);
+        return e | ((od << 3) & 0x70707070u) | (od & 0x80808080u);
+    }
+    // bit 7 of byte j -> bit 2j of the top byte
+    const uint32_t se = (((ev >> 7) & 0x01010101u) * 0x01041040u) >> 24, so = (((od >> 7) & 0x01010101u) * 0x01041040u) >> 24;
+    sbits = (se & 0x55u) | ((so & 0x55u) << 1);
+    return (ev & 0x0F0F0F0Fu) | ((od & 0x0F0F0F0Fu) << 4);
+}
+
 // The C chunks of one thread-unit, after the block scale is known.  SMALL: see chunk_errors (warp-uniform).
 // On return xb[k] holds chunk k's fake-quantised values (fp16 pairs with the inputs' signs), `bests` the chosen
 // candidate of every chunk (2 bits each) and the return value is the packed minimum of all quotients a.
@@ -126,7 +164,7 @@ __device__ __forceinline__ int first_min4(const float* acc)
 template <int MB, int C, int ML, bool SMALL, bool SIDE, int TINY>
 __device__ __forceinline__ uint32_t unit_chunks(const TabArgs& a, const uint32_t tab_addr, const uint32_t* s_nt2,
                                                  const float* s_tabf, uint32_t (*xb)[4], uint32_t l1b, const uint4 cst,
-                                                 int m_lanes, uint32_t& bests, uint32_t (*cwout)[4])
+                                                 int m_lanes, uint32_t& bests, uint32_t* codes, uint32_t* sbits)
 {
     const __half2 pre2 = bits_h2(cst.x), post2 = bits_h2(cst.y), nm2 = bits_h2(cst.z), rm2 = bits_h2(cst.w);
     const uint32_t l1u = l1b * 0x00010001u;
@@ -178,15 +216,16 @@ __device__ __forceinline__ uint32_t unit_chunks(const TabArgs& a, const uint32_t
         const uint32_t wsel = 0x4C08u + (uint32_t)best * 0x1111u;
         const uint32_t ntb = s_nt2[best];
         const __half2 tlb = __hmul2(bits_h2(l1u), bits_h2(ntb));
-        uint32_t dq[4];
+        uint32_t dq[4], cwv[SIDE ? 4 : 1];
         #pragma unroll
         for (int p = 0; p < 4; ++p) {
             const uint32_t cw = prmt(ent[2 * p], ent[2 * p + 1], wsel);
-            if (SIDE) cwout[k][p] = cw;
+            if (SIDE) cwv[p] = cw;
             const __half2 dneg = SMALL ? __hmul2(bits_h2(cw), tlb)
                                        : __hmul2(__hmul2(bits_h2(cw), bits_h2(ntb)), bits_h2(l1u));
             dq[p] = (h2_bits(dneg) & 0x7FFF7FFFu) | (xb[k][p] & 0x80008000u);
         }
+        if (SIDE) codes[k] = pack_codes<MB>(cwv, xb[k], sbits[k]);
         if (TINY == 1) {
             const __half2 am = __hmin2(__hmin2(bits_h2(av[0]), bits_h2(av[1])), __hmin2(bits_h2(av[2]), bits_h2(av[3])));
             if (__hle2_mask(am, bits_h2(0x00200020u)) != 0u) {
@@ -212,23 +251,28 @@ __device__ __forceinline__ uint32_t unit_chunks(const TabArgs& a, const uint32_t
 // Stage a format's tables into shared memory; every thread of the CTA calls it.  The candidate table comes
 // by ONE bulk async copy whose completion is counted on an mbarrier, with a bounded wait: if the copy has not
 // landed by then, every thread loads the table with plain loads (the same values, so a late completion of the
-// copy is harmless).  Returns the shared-memory address of the table.
+// copy is harmless).  MIX: the second table follows the first.  Returns the shared-memory address of the first table.
+template <bool MIX = false>
 __device__ __forceinline__ uint32_t stage_table(const TabArgs& a, uint32_t* s_tab, uint4* s_l1c, unsigned long long* s_bar,
                                                  uint32_t* s_nt2, float* s_tabf, int nthreads)
 {
     const int tid = threadIdx.x;
     if (tid < 4) { s_nt2[tid] = a.nt2[tid]; s_tabf[tid] = a.tabf[tid]; }
+    if (MIX && tid >= 4 && tid < 8) { s_nt2[tid] = a.b.nt2[tid - 4]; s_tabf[tid] = a.b.tabf[tid - 4]; }
     const uint32_t bar = smem_addr(s_bar), dst = smem_addr(s_tab);
-    const uint32_t bytes = (uint32_t)a.entries * 4u;
+    const uint32_t bytes = (uint32_t)a.entries * 4u, bytes1 = MIX ? (uint32_t)a.b.entries * 4u : 0u;
     if (tid == 0) {
         asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(bar));
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
     __syncthreads();
     if (tid == 0) {
-        asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(bytes) : "memory");
+        asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(bytes + bytes1) : "memory");
         asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];"
                      ::"r"(dst), "l"(a.table), "r"(bytes), "r"(bar) : "memory");
+        if (MIX)
+            asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];"
+                         ::"r"(dst + bytes), "l"(a.b.table), "r"(bytes1), "r"(bar) : "memory");
     }
     if (tid < 256) {
         const uint32_t l1b = (uint32_t)tid << 7;
@@ -253,6 +297,10 @@ __device__ __forceinline__ uint32_t stage_table(const TabArgs& a, uint32_t* s_ta
         const uint4* src = reinterpret_cast<const uint4*>(a.table);
         uint4* d4 = reinterpret_cast<uint4*>(s_tab);
         for (int i = tid; i < a.entries / 4; i += nthreads) d4[i] = __ldg(src + i);
+        if (MIX) {
+            const uint4* src1 = reinterpret_cast<const uint4*>(a.b.table);
+            for (int i = tid; i < a.b.entries / 4; i += nthreads) d4[a.entries / 4 + i] = __ldg(src1 + i);
+        }
         __syncthreads();
     }
     return dst;
@@ -275,6 +323,40 @@ __device__ __forceinline__ uint32_t unit_scale(const uint32_t (*xb)[4], int Gt, 
     uint32_t sb = (uint32_t)h_bits(__float2half_rn(sf));
     sb = min(max(sb, 0x0400u), 0x7B80u);
     return (sb + 0x40u) & 0xFF80u;
+}
+
+// The E5M3 scale's fp16 pattern for a block whose maximum divided by the largest element value is `sf`.
+__device__ __forceinline__ uint32_t e5m3_scale(float sf)
+{
+    const uint32_t sb = min(max((uint32_t)h_bits(__float2half_rn(sf)), 0x0400u), 0x7B80u);
+    return (sb + 0x40u) & 0xFF80u;
+}
+
+// A block's error total from its chunks' sums (chunk g + k * Gt of lane g): the tree of an exchange between lanes
+// that hold one chunk each, distances 8, 4, 2, 1 (16 chunks), with the distances of Gt and more inside the thread.
+template <int C>
+__device__ __forceinline__ float block_error(const float* e, int Gt)
+{
+    float t = C == 4 ? (e[0] + e[2]) + (e[1] + e[3]) : e[0] + e[1];
+    for (int off = Gt >> 1; off >= 1; off >>= 1) t += __shfl_xor_sync(0xFFFFFFFFu, t, off);
+    return t;
+}
+
+// The per-block side outputs, by the block's first lane (`store`); l2word: this lane's share of the micro-scale indices.
+__device__ __forceinline__ void store_block_side(const TabArgs& a, int64_t bi, int Gt, bool store, uint32_t l1b, uint32_t scheme,
+                                                 uint32_t l2word)
+{
+    if (a.out.l2_packed) l2word = group_or(l2word, Gt);
+    if (!store) return;
+    if (a.out.scale_h) a.out.scale_h[bi] = (uint16_t)l1b;
+    if (a.out.scale_u8) a.out.scale_u8[bi] = (uint8_t)(l1b >> 7);
+    if (a.out.scheme) a.out.scheme[bi] = (uint8_t)scheme;
+    if (a.out.l2_packed) {
+        uint8_t* lp = a.out.l2_packed + bi * a.l2_bytes;
+        if (a.l2_bytes == 4) *reinterpret_cast<uint32_t*>(lp) = l2word;
+        else if (a.l2_bytes == 2) *reinterpret_cast<uint16_t*>(lp) = (uint16_t)l2word;
+        else *lp = (uint8_t)l2word;
+    }
 }
 
 // GT / ML: lanes per block / per micro-block as compile-time constants (0: read from the arguments).
@@ -362,11 +444,11 @@ __global__ void __launch_bounds__(TAB_THREADS, 2) hbq_tab_kernel(const TabArgs a
 
         // ---- the chunks: candidates' errors, choice, values ----
         uint32_t bests, amin;
-        uint32_t cw[SIDE ? C : 1][4];
+        uint32_t codes[SIDE ? C : 1], sbits[SIDE ? C : 1];
         // value * t * l1 overflows fp16 only for blocks whose maximum is within 1 % of fp16's own: one
         // warp-uniform branch between the fused form and the form that keeps each product's rounding
-        if (__all_sync(0xFFFFFFFFu, l1b < a.big_l1)) amin = unit_chunks<MB, C, ML, true, SIDE, 0>(a, dst, s_nt2, s_tabf, xb, l1b, cst, a.m_lanes, bests, cw);
-        else amin = unit_chunks<MB, C, ML, false, SIDE, 0>(a, dst, s_nt2, s_tabf, xb, l1b, cst, a.m_lanes, bests, cw);
+        if (__all_sync(0xFFFFFFFFu, l1b < a.big_l1)) amin = unit_chunks<MB, C, ML, true, SIDE, 0>(a, dst, s_nt2, s_tabf, xb, l1b, cst, a.m_lanes, bests, codes, sbits);
+        else amin = unit_chunks<MB, C, ML, false, SIDE, 0>(a, dst, s_nt2, s_tabf, xb, l1b, cst, a.m_lanes, bests, codes, sbits);
 
         // The reference returns +0 (not -0) when fp16(a / t) is exactly zero.  Only quotients a below 2^-19
         // can do that; deciding it needs the exact a, where the scaled division may be off: rare, so the
@@ -397,7 +479,11 @@ __global__ void __launch_bounds__(TAB_THREADS, 2) hbq_tab_kernel(const TabArgs a
                         const uint32_t xbits = (xr[p] >> (16 * h)) & 0xFFFFu;
                         if (xbits & 0x8000u) {
                             const float xf = __half2float(bits_h((uint16_t)(xbits & 0x7FFFu)));
-                            if (rh(__fdiv_rn(rh(__fdiv_rn(xf, l1f)), tc)) == 0.f) xb[k][p] &= ~(0x8000u << (16 * h));
+                            if (rh(__fdiv_rn(rh(__fdiv_rn(xf, l1f)), tc)) == 0.f) {
+                                xb[k][p] &= ~(0x8000u << (16 * h));
+                                if (SIDE && MB == 1) codes[k] &= ~(8u << (4 * (2 * p + h)));
+                                if (SIDE && MB == 2) sbits[k] &= ~(1u << (2 * p + h));
+                            }
                         }
                     }
             }
@@ -414,25 +500,15 @@ __global__ void __launch_bounds__(TAB_THREADS, 2) hbq_tab_kernel(const TabArgs a
                 const int mbi = cib >> a.log2m;                  // its micro-block
                 const bool leader = (g & (a.m_lanes - 1)) == 0;
                 if (valid && a.out.codes) {
-                    uint32_t wcode = 0u, sbits = 0u;
-                    #pragma unroll
-                    for (int p = 0; p < 4; ++p) {
-                        const uint32_t mag = code2_e2<MB>(bits_h2(cw[k][p]));
-                        uint32_t lo = mag & 0xFFFFu, hi = mag >> 16;
-                        const uint32_t slo = (xb[k][p] >> 15) & 1u, shi = xb[k][p] >> 31;
-                        if (MB == 1) { lo |= slo << 3; hi |= shi << 3; }
-                        wcode |= ((lo & 0xFu) | ((hi & 0xFu) << 4)) << (8 * p);
-                        sbits |= (slo | (shi << 1)) << (2 * p);
-                    }
-                    reinterpret_cast<uint32_t*>(a.out.codes)[ci] = wcode;
-                    if (MB == 2 && a.out.sign) a.out.sign[ci] = (uint8_t)sbits;
+                    reinterpret_cast<uint32_t*>(a.out.codes)[ci] = codes[k];
+                    if (MB == 2 && a.out.sign) a.out.sign[ci] = (uint8_t)sbits[k];
                 }
                 if (leader) {
                     if (a.out.l2_packed) l2word |= (uint32_t)best << (mbi * a.l2_sc_bit);
                     if (valid && a.out.l2_idx) a.out.l2_idx[bi * a.nl2 + mbi] = (uint8_t)best;
                 }
             }
-            if (valid) {
+            if (valid && (!SIDE || a.deq)) {
                 uint32_t dq[4] = {xb[k][0], xb[k][1], xb[k][2], xb[k][3]};
                 if (a.out_bf16) {
                     #pragma unroll
@@ -445,20 +521,196 @@ __global__ void __launch_bounds__(TAB_THREADS, 2) hbq_tab_kernel(const TabArgs a
                 a.deq[ci] = make_uint4(dq[0], dq[1], dq[2], dq[3]);
             }
         }
-        if (SIDE) {
-            if (a.out.l2_packed) l2word = group_or(l2word, Gt);
-            if (valid && g == 0) {
-                if (a.out.scale_h) a.out.scale_h[bi] = (uint16_t)l1b;
-                if (a.out.scale_u8) a.out.scale_u8[bi] = (uint8_t)(l1b >> 7);
-                if (a.out.scheme) a.out.scheme[bi] = 0;
-                if (a.out.l2_packed) {
-                    uint8_t* lp = a.out.l2_packed + bi * a.l2_bytes;
-                    if (a.l2_bytes == 4) *reinterpret_cast<uint32_t*>(lp) = l2word;
-                    else if (a.l2_bytes == 2) *reinterpret_cast<uint16_t*>(lp) = (uint16_t)l2word;
-                    else *lp = (uint8_t)l2word;
-                }
+        if (SIDE) store_block_side(a, bi, Gt, valid && g == 0, l1b, 0u, l2word);
+    }
+}
+
+
+// ---- the two-table ("Mix") weight formats ----------------------------------------------------------------------
+// Both candidate tables are evaluated, each with its own block scale; the one with the smaller fp16 total of the chosen
+// candidates' squared errors over the block wins, the first on ties (src/quantizer.py:806-840).  Per scheme a chunk
+// leaves its chosen candidate (2 bits), its eight winning value bytes (two registers) and its error sum, so that after
+// the comparison only the values are formed: the division, the lookups and the candidates' errors are paid twice,
+// everything else once.  The totals are added in the order of the tree over the block's chunks that the other kernels
+// use (chunk distance 8, 4, 2, 1), so a sum that the fp32 additions round is the same number in all of them.
+// Bound: instruction issue (about twice hbq_tab_kernel's work per element).  Weight [14336, 4096] to packed planes:
+// 136 us; the arithmetic kernel of quantize.cu, which alone had these outputs, took 507 us.
+template <int MB, int C, int ML, bool SMALL>
+__device__ __forceinline__ void scheme_chunks(const uint32_t tab_addr, uint32_t base2, uint32_t hi2, uint32_t entry_bytes,
+                                              const uint32_t* nt2, const uint32_t (*xb)[4], uint32_t l1b, const uint4 cst,
+                                              int m_lanes, uint32_t& bests, uint32_t (*win)[2], float* err, uint32_t& amin)
+{
+    const __half2 pre2 = bits_h2(cst.x), post2 = bits_h2(cst.y), nm2 = bits_h2(cst.z), rm2 = bits_h2(cst.w);
+    const uint32_t l1u = l1b * 0x00010001u;
+    uint32_t tl[4];
+    #pragma unroll
+    for (int i = 0; i < 4; ++i) tl[i] = h2_bits(__hmul2(bits_h2(l1u), bits_h2(nt2[i])));
+    bests = 0u;
+    amin = 0x7C007C00u;
+    const uint32_t addr0 = tab_addr - 4u * (base2 & 0xFFFFu);
+    #pragma unroll
+    for (int k = 0; k < C; ++k) {
+        uint32_t ent[8];
+        #pragma unroll
+        for (int p = 0; p < 4; ++p) {
+            const __half2 axs = __hmul2(__habs2(bits_h2(xb[k][p])), pre2);
+            const __half2 q0 = __hmul2(axs, rm2);
+            const __half2 r = __hfma2(q0, nm2, axs);
+            const __half2 aa = __hmul2(__hfma2(r, rm2, q0), post2);
+            amin = h2_bits(__hmin2(bits_h2(amin), aa));
+            const uint32_t w = h2_bits(__hmin2(__hmax2(aa, bits_h2(base2)), bits_h2(hi2)));
+            asm volatile("ld.shared.u32 %0, [%1];" : "=r"(ent[2 * p]) : "r"((w & 0xFFFFu) * entry_bytes + addr0));
+            asm volatile("ld.shared.u32 %0, [%1];" : "=r"(ent[2 * p + 1]) : "r"((w >> 16) * entry_bytes + addr0));
+        }
+        float own[4], acc[4];
+        chunk_errors<SMALL>(ent, xb[k], tl, nt2, l1u, own);
+        #pragma unroll
+        for (int i = 0; i < 4; ++i) acc[i] = own[i];
+        if (ML > 0) {
+            #pragma unroll
+            for (int off = ML >> 1; off >= 1; off >>= 1) {
+                #pragma unroll
+                for (int i = 0; i < 4; ++i) acc[i] += __shfl_xor_sync(0xFFFFFFFFu, acc[i], off);
+            }
+        } else {
+            for (int off = m_lanes >> 1; off >= 1; off >>= 1) {
+                #pragma unroll
+                for (int i = 0; i < 4; ++i) acc[i] += __shfl_xor_sync(0xFFFFFFFFu, acc[i], off);
             }
         }
+        const uint32_t best = (uint32_t)first_min4(acc);
+        bests |= best << (2 * k);
+        const float e01 = (best & 1u) ? own[1] : own[0], e23 = (best & 1u) ? own[3] : own[2];
+        err[k] = (best & 2u) ? e23 : e01;
+        const uint32_t sel = best * 0x11u + 0x40u;              // byte `best` of both operands
+        win[k][0] = prmt(prmt(ent[0], ent[1], sel), prmt(ent[2], ent[3], sel), 0x5410u);
+        win[k][1] = prmt(prmt(ent[4], ent[5], sel), prmt(ent[6], ent[7], sel), 0x5410u);
+    }
+}
+
+template <int MB, int GT, int ML, bool SIDE>
+__global__ void __launch_bounds__(MIX_THREADS, 2) hbq_tab_mix_kernel(const TabArgs a)
+{
+    constexpr int C = 4;
+    extern __shared__ __align__(128) uint32_t s_tab[];
+    __shared__ uint4 s_l1c[256];
+    __shared__ __align__(8) unsigned long long s_bar;
+    __shared__ uint32_t s_nt2[8];
+    __shared__ float s_tabf[8];
+    const int tid = threadIdx.x, lane = tid & 31;
+    const uint32_t dst = stage_table<true>(a, s_tab, s_l1c, &s_bar, s_nt2, s_tabf, MIX_THREADS);
+    const int log2Gt = GT == 4 ? 2 : a.log2Gt;
+    const int Gt = 1 << log2Gt;
+    const int64_t stride = (int64_t)gridDim.x * MIX_THREADS;
+
+    #pragma unroll 1
+    for (int64_t u = (int64_t)blockIdx.x * MIX_THREADS + tid; u - lane < a.total_units; u += stride) {
+        const bool valid = u < a.total_units;
+        const int64_t bi = u >> log2Gt;
+        const int g = (int)u & (Gt - 1);
+        const int64_t c0 = bi * (int64_t)(C * Gt) + g;
+        uint32_t xb[C][4];
+        #pragma unroll
+        for (int k = 0; k < C; ++k) {
+            const uint4 r = valid ? __ldg(a.x + c0 + k * Gt) : make_uint4(0u, 0u, 0u, 0u);
+            xb[k][0] = r.x; xb[k][1] = r.y; xb[k][2] = r.z; xb[k][3] = r.w;
+        }
+        if (a.in_bf16) {
+            #pragma unroll
+            for (int k = 0; k < C; ++k)
+                #pragma unroll
+                for (int p = 0; p < 4; ++p)
+                    xb[k][p] = h2_bits(__floats2half2_rn(__uint_as_float(xb[k][p] << 16), __uint_as_float(xb[k][p] & 0xFFFF0000u)));
+        }
+        // the block maximum serves both schemes; their scales differ by the largest candidate
+        uint32_t mx = 0u;
+        #pragma unroll
+        for (int k = 0; k < C; ++k)
+            #pragma unroll
+            for (int p = 0; p < 4; ++p) mx = h2_bits(__hmax2(bits_h2(mx), __habs2(bits_h2(xb[k][p]))));
+        for (int off = Gt >> 1; off >= 1; off >>= 1)
+            mx = h2_bits(__hmax2(bits_h2(mx), bits_h2(__shfl_xor_sync(0xFFFFFFFFu, mx, off))));
+        const float amax = __half2float(bits_h((uint16_t)max(mx & 0xFFFFu, mx >> 16)));
+        const uint32_t l1a = e5m3_scale(amax * a.inv_ele_max), l1c = e5m3_scale(amax * a.b.inv_ele_max);
+
+        uint32_t bests, bests1, win[C][2], win1[C][2], amin, amin1;
+        float err[C], err1[C];
+        const bool small = __all_sync(0xFFFFFFFFu, l1a < a.big_l1 && l1c < a.b.big_l1);
+        if (small) scheme_chunks<MB, C, ML, true>(dst, a.base2, a.hi2, a.entry_bytes, a.nt2, xb, l1a, s_l1c[l1a >> 7], a.m_lanes, bests, win, err, amin);
+        else scheme_chunks<MB, C, ML, false>(dst, a.base2, a.hi2, a.entry_bytes, a.nt2, xb, l1a, s_l1c[l1a >> 7], a.m_lanes, bests, win, err, amin);
+        const float tot = block_error<C>(err, Gt);
+        const uint32_t dst1 = dst + (uint32_t)a.entries * 4u;
+        if (small) scheme_chunks<MB, C, ML, true>(dst1, a.b.base2, a.b.hi2, a.entry_bytes, a.b.nt2, xb, l1c, s_l1c[l1c >> 7], a.m_lanes, bests1, win1, err1, amin1);
+        else scheme_chunks<MB, C, ML, false>(dst1, a.b.base2, a.b.hi2, a.entry_bytes, a.b.nt2, xb, l1c, s_l1c[l1c >> 7], a.m_lanes, bests1, win1, err1, amin1);
+        const float tot1 = block_error<C>(err1, Gt);
+        const bool second = rh(tot1) < rh(tot);                  // the same in every lane of the block
+        if (second) {
+            bests = bests1; amin = amin1;
+            #pragma unroll
+            for (int k = 0; k < C; ++k) { win[k][0] = win1[k][0]; win[k][1] = win1[k][1]; }
+        }
+        const uint32_t l1b = second ? l1c : l1a, sidx = second ? 4u : 0u;
+        const uint32_t l1u = l1b * 0x00010001u;
+        const float l1f = __half2float(bits_h((uint16_t)l1b));
+        const bool tiny = __hle2_mask(bits_h2(amin), bits_h2(0x00200020u)) != 0u;
+
+        uint32_t l2word = 0u;
+        #pragma unroll
+        for (int k = 0; k < C; ++k) {
+            const int64_t ci = c0 + k * Gt;
+            const uint32_t best = (bests >> (2 * k)) & 3u;
+            const uint32_t nt = s_nt2[sidx + best];
+            const __half2 tlb = __hmul2(bits_h2(l1u), bits_h2(nt));
+            uint32_t cw[4], sg[4], dq[4];
+            #pragma unroll
+            for (int p = 0; p < 4; ++p) {
+                cw[p] = prmt(win[k][p >> 1], 0u, (p & 1) ? 0x3424u : 0x1404u);       // value bytes -> fp16 pair
+                sg[p] = xb[k][p] & 0x80008000u;
+            }
+            if (tiny) {                                          // the reference's +0 where fp16(a / t) is zero (see unit_chunks)
+                const float tc = s_tabf[sidx + best];
+                #pragma unroll
+                for (int p = 0; p < 4; ++p)
+                    #pragma unroll
+                    for (int h = 0; h < 2; ++h) {
+                        const uint32_t xbits = (xb[k][p] >> (16 * h)) & 0xFFFFu;
+                        if (xbits & 0x8000u) {
+                            const float xf = __half2float(bits_h((uint16_t)(xbits & 0x7FFFu)));
+                            if (rh(__fdiv_rn(rh(__fdiv_rn(xf, l1f)), tc)) == 0.f) sg[p] &= ~(0x8000u << (16 * h));
+                        }
+                    }
+            }
+            #pragma unroll
+            for (int p = 0; p < 4; ++p) {
+                const __half2 dneg = small ? __hmul2(bits_h2(cw[p]), tlb) : __hmul2(__hmul2(bits_h2(cw[p]), bits_h2(nt)), bits_h2(l1u));
+                dq[p] = (h2_bits(dneg) & 0x7FFF7FFFu) | sg[p];
+            }
+            if (SIDE) {
+                const int mbi = (g + k * Gt) >> a.log2m;
+                const bool leader = (g & (a.m_lanes - 1)) == 0;
+                if (valid && a.out.codes) {
+                    uint32_t sb = 0u;
+                    reinterpret_cast<uint32_t*>(a.out.codes)[ci] = pack_codes<MB>(cw, sg, sb);
+                    if (MB == 2 && a.out.sign) a.out.sign[ci] = (uint8_t)sb;
+                }
+                if (leader) {
+                    if (a.out.l2_packed) l2word |= best << (mbi * a.l2_sc_bit);
+                    if (valid && a.out.l2_idx) a.out.l2_idx[bi * a.nl2 + mbi] = (uint8_t)best;
+                }
+            }
+            if (valid && a.deq) {
+                if (a.out_bf16) {
+                    #pragma unroll
+                    for (int p = 0; p < 4; ++p) {
+                        const float2 f = __half22float2(bits_h2(dq[p]));
+                        const __nv_bfloat162 bb = __floats2bfloat162_rn(f.x, f.y);
+                        dq[p] = *reinterpret_cast<const uint32_t*>(&bb);
+                    }
+                }
+                a.deq[ci] = make_uint4(dq[0], dq[1], dq[2], dq[3]);
+            }
+        }
+        if (SIDE) store_block_side(a, bi, Gt, valid && g == 0, l1b, second ? 1u : 0u, l2word);
     }
 }
 
@@ -735,10 +987,10 @@ __global__ void __launch_bounds__(ROW_THREADS, 2) hbq_row_kernel(const RowArgs a
                 const uint32_t l1b = unit_scale<4>(xb, 4, a.t.inv_ele_max);
                 const uint4 cst = s_l1c[l1b >> 7];
                 uint32_t bests;
-                uint32_t cw[1][4];
+                uint32_t nocodes[1], nosigns[1];
                 constexpr int TINY = PRO == ROW_SOFTMAX ? 2 : 1;
-                if (__all_sync(0xFFFFFFFFu, l1b < a.t.big_l1)) unit_chunks<MB, 4, ML, true, false, TINY>(a.t, dst, s_nt2, s_tabf, xb, l1b, cst, ML, bests, cw);
-                else unit_chunks<MB, 4, ML, false, false, TINY>(a.t, dst, s_nt2, s_tabf, xb, l1b, cst, ML, bests, cw);
+                if (__all_sync(0xFFFFFFFFu, l1b < a.t.big_l1)) unit_chunks<MB, 4, ML, true, false, TINY>(a.t, dst, s_nt2, s_tabf, xb, l1b, cst, ML, bests, nocodes, nosigns);
+                else unit_chunks<MB, 4, ML, false, false, TINY>(a.t, dst, s_nt2, s_tabf, xb, l1b, cst, ML, bests, nocodes, nosigns);
             }
             if (valid) {
                 #pragma unroll
@@ -803,6 +1055,27 @@ static int launch_tab_variant(const TabArgs& a, bool side, bool glu, size_t smem
     if (glu) return launch_tab<MB, C, GT, ML, false, true>(a, smem, stream);
     if (side) return launch_tab<MB, C, GT, ML, true, false>(a, smem, stream);
     return launch_tab<MB, C, GT, ML, false, false>(a, smem, stream);
+}
+
+template <int MB, int GT, int ML, bool SIDE>
+static int launch_mix(const TabArgs& a, size_t smem, cudaStream_t stream)
+{
+    int sms = 0, per_sm = 0;
+    { const int rc = device_sms(&sms); if (rc) return rc; }
+    { const int rc = ensure_dynamic_smem(hbq_tab_mix_kernel<MB, GT, ML, SIDE>, smem); if (rc) return rc; }
+    { const int rc = resident_ctas(hbq_tab_mix_kernel<MB, GT, ML, SIDE>, MIX_THREADS, smem, &per_sm); if (rc) return rc; }
+    const int64_t need = (a.total_units + MIX_THREADS - 1) / MIX_THREADS, cap = (int64_t)sms * per_sm;
+    hbq_tab_mix_kernel<MB, GT, ML, SIDE><<<(int)(need < cap ? need : cap), MIX_THREADS, smem, stream>>>(a);
+    HBQ_LAUNCH_CHECK("hbq_tab_mix_kernel");
+    return HBQ_OK;
+}
+
+template <int MB>
+static int launch_mix_geometry(const TabArgs& a, int Gt, int m, bool side, size_t smem, cudaStream_t stream)
+{
+    if (Gt == 4 && m == 1) return side ? launch_mix<MB, 4, 1, true>(a, smem, stream) : launch_mix<MB, 4, 1, false>(a, smem, stream);
+    if (Gt == 4 && m == 4) return side ? launch_mix<MB, 4, 4, true>(a, smem, stream) : launch_mix<MB, 4, 4, false>(a, smem, stream);
+    return side ? launch_mix<MB, 0, 0, true>(a, smem, stream) : launch_mix<MB, 0, 0, false>(a, smem, stream);
 }
 
 // The shipped configurations (block 128: 4 chunks per thread, 4 lanes per block; micro-block 8 or 32) have
@@ -934,13 +1207,14 @@ int softmax_quantize_launch(const void* scores, int64_t rows, int64_t S, int64_t
 int hbq_tab_try_launch(const QArgs& q, int mb, cudaStream_t stream, bool* launched)
 {
     *launched = false;
-    if (mb < 1 || mb > 2 || q.nscheme != 1 || q.nc > 4 || !q.scale_fast_e5m3) return HBQ_OK;
-    if (!q.deq || !q.aligned || q.K != q.Kp) return HBQ_OK;
+    if (mb < 1 || mb > 2 || q.nscheme > 2 || q.nc > 4 || !q.scale_fast_e5m3) return HBQ_OK;
+    if (!q.aligned || q.K != q.Kp) return HBQ_OK;
     if (q.rope_cos || q.perm_T > 0 || q.k_center) return HBQ_OK;
     const bool side = q.out.codes || q.out.sign || q.out.scale_u8 || q.out.scale_h || q.out.l2_packed || q.out.l2_idx ||
                       q.out.scheme;
-    const bool glu = q.glu_gate != nullptr;
-    if (glu && (side || q.in_bf16 || q.out_bf16)) return HBQ_OK;
+    const bool glu = q.glu_gate != nullptr, mix = q.nscheme == 2;
+    if (!side && !q.deq) return HBQ_OK;
+    if (glu && (mix || side || q.in_bf16 || q.out_bf16)) return HBQ_OK;
     if ((reinterpret_cast<uintptr_t>(q.out.codes) & 3) || (reinterpret_cast<uintptr_t>(q.out.l2_packed) & 3) ||
         (reinterpret_cast<uintptr_t>(q.out.scale_h) & 1))
         return HBQ_OK;
@@ -950,34 +1224,34 @@ int hbq_tab_try_launch(const QArgs& q, int mb, cudaStream_t stream, bool* launch
     int C = 0;
     if (cpb % 4 == 0 && m <= cpb / 4) C = 4;
     else if (cpb % 2 == 0 && m <= cpb / 2) C = 2;
-    if (C == 0) return HBQ_OK;
+    if (C == 0 || (mix && C != 4)) return HBQ_OK;
     const int Gt = cpb / C;
     if (Gt > 32 || (Gt & (Gt - 1)) || (m & (m - 1))) return HBQ_OK;
 
-    TabTable t;
-    if (!hbq_tab_table(mb, q.tab[0], q.nc, &t) || t.slot >= TAB_SLOTS || t.entries > TAB_MAX_ENTRIES) return HBQ_OK;
     TabArgs a;
-    memset(&a, 0, sizeof(a));
-    { const int rc = table_on_device(t, stream, &a.table); if (rc) return rc; }
-    if (!a.table) return HBQ_OK;
+    bool ok = false;
+    { const int rc = fill_format(q, mb, stream, &a, &ok); if (rc) return rc; }
+    if (!ok) return HBQ_OK;
+    if (mix) {                                               // the second table, through the same steps
+        QArgs q2;
+        memset(&q2, 0, sizeof(q2));
+        memcpy(q2.tab[0], q.tab[1], sizeof(q2.tab[0]));
+        q2.nc = q.nc;
+        q2.ele_max[0] = q.ele_max[1];
+        TabArgs b;
+        { const int rc = fill_format(q2, mb, stream, &b, &ok); if (rc) return rc; }
+        if (!ok) return HBQ_OK;
+        a.b.table = b.table; a.b.entries = b.entries;
+        a.b.base2 = b.base2; a.b.hi2 = b.hi2; a.b.big_l1 = b.big_l1; a.b.inv_ele_max = b.inv_ele_max;
+        memcpy(a.b.nt2, b.nt2, sizeof(b.nt2));
+        memcpy(a.b.tabf, b.tabf, sizeof(b.tabf));
+    }
 
     a.x = reinterpret_cast<const uint4*>(q.x);
     a.gate = reinterpret_cast<const uint4*>(q.glu_gate);
     a.deq = reinterpret_cast<uint4*>(q.deq);
     a.out = q.out;
     a.total_units = q.total_chunks / C;
-    a.entries = t.entries;
-    a.entry_bytes = 4u;
-    a.base2 = (uint32_t)t.base * 0x00010001u;
-    a.hi2 = (uint32_t)t.hi * 0x00010001u;
-    a.big_l1 = t.big_l1;
-    a.inv_ele_max = 1.f / q.ele_max[0];
-    for (int i = 0; i < 4; ++i) {
-        const float tv = q.tab[0][i < q.nc ? i : q.nc - 1];     // unused slots repeat the last candidate: they never win a tie
-        a.tabf[i] = tv;
-        a.nt2[i] = (uint32_t)__half_as_ushort(__float2half_rn(-tv)) * 0x00010001u;
-    }
-    memcpy(a.rm, t.rm, sizeof(a.rm));
     a.in_bf16 = q.in_bf16; a.out_bf16 = q.out_bf16;
     while ((1 << a.log2Gt) < Gt) ++a.log2Gt;
     a.m_lanes = m;
@@ -986,9 +1260,11 @@ int hbq_tab_try_launch(const QArgs& q, int mb, cudaStream_t stream, bool* launch
     a.nl2 = q.f.block_size / L;
     a.l2_bytes = (a.nl2 * a.l2_sc_bit) >> 3;
 
-    const size_t smem = (size_t)t.entries * 4;
-    const int rc = mb == 1 ? launch_tab_geometry<1>(a, C, Gt, m, side, glu, smem, stream)
-                           : launch_tab_geometry<2>(a, C, Gt, m, side, glu, smem, stream);
+    const size_t smem = (size_t)(a.entries + (mix ? a.b.entries : 0)) * 4;
+    int rc;
+    if (mix) rc = mb == 1 ? launch_mix_geometry<1>(a, Gt, m, side, smem, stream) : launch_mix_geometry<2>(a, Gt, m, side, smem, stream);
+    else rc = mb == 1 ? launch_tab_geometry<1>(a, C, Gt, m, side, glu, smem, stream)
+                      : launch_tab_geometry<2>(a, C, Gt, m, side, glu, smem, stream);
     if (rc == HBQ_OK) *launched = true;
     return rc;
 }
