@@ -55,3 +55,27 @@ def test_mix_outputs_match_the_oracle(oracle, block, micro, mb, rows, dtype):
             assert np.array_equal(np.unpackbits(packed.sign.cpu().numpy(), axis=-1, bitorder="little"), oc >> 4)
         assert np.array_equal(packed.scheme.cpu().numpy(), o["scheme"])
         assert torch.equal(H.dequantize_packed(packed).cpu().view(torch.int16), want.view(torch.int16))
+
+
+@pytest.mark.parametrize("block,micro,mb", [(128, 8, 1), (128, 32, 2), (32, 8, 1)])
+def test_mix_packed_outputs_of_infinite_and_nan_inputs(oracle, block, micro, mb):
+    """An infinity takes the largest element value in every packed output and a NaN stays one in the tensor, as in the
+    oracle (which leaves a NaN's code open)."""
+    import hbq_b200 as H
+    x = _inputs(41, 1536, 5)
+    rng = np.random.default_rng(6)
+    x[rng.random(x.shape) < 0.004] = np.float16(np.inf)
+    x[rng.random(x.shape) < 0.004] = np.float16(-np.inf)
+    x[3, :block] = np.float16(np.inf)
+    x[rng.random(x.shape) < 0.002] = np.float16(np.nan)
+    x[5, :block] = np.float16(np.nan)
+    ok = ~np.isnan(x)
+    o = oracle.quantize(x, oracle.Format(oracle.KIND_HBQ, 2, mb, 5, 3, block, l2_block_size=micro, l2_sc_bit=2, l2_scheme="Mix"))
+    q = H.HBQQuantizer(block_size=block, ebit=2, mbit=mb, sc_ebit=5, sc_mbit=3, l2_block_size=micro, l2_sc_bit=2, l2_scheme="Mix")
+    packed, deq = q.quantize_packed(torch.from_numpy(x).cuda(), with_deq=True)
+    pc = packed.codes.cpu().numpy()
+    un = np.stack([pc & 0xF, pc >> 4], axis=-1).reshape(41, -1)
+    assert np.array_equal(un[ok], o["codes"].reshape(41, -1).astype(np.uint8)[ok] & 0xF)
+    assert np.array_equal(packed.scheme.cpu().numpy(), o["scheme"])
+    got = deq.cpu().numpy()
+    assert np.array_equal(bits(got)[ok], bits(o["deq"].reshape(41, -1))[ok]) and np.isnan(got[~ok]).all()
