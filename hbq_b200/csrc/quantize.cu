@@ -960,8 +960,13 @@ int quantize_launch(const void* x, int dtype, int64_t rows, int64_t K, const hbq
         const int tb = (B / L) * f->l2_sc_bit;
         if (tb != 8 && tb != 16 && tb != 32) return HBQ_ERR_UNSUPPORTED;
     }
-    if (kv && kv->v_axis)
+    if (kv && kv->v_axis) {
+        bool launched = false;
+        const int rc = hbq_tab_v_try_launch(a, fast_mb, x, deq, a.in_bf16, a.out_bf16, kv->B, kv->T, kv->H, kv->D, kv->v_out_token_major,
+                                            stream, &launched);
+        if (rc != HBQ_OK || launched) return rc;
         return hbq_lut_v_launch(a, fast_mb, x, deq, a.in_bf16, a.out_bf16, kv->B, kv->T, kv->H, kv->D, kv->v_out_token_major, stream);
+    }
     {
         bool launched = false;
         int rc = hbq_tab_try_launch(a, fast_mb, stream, &launched);          // byte-table kernels (quantize_tab.cu)

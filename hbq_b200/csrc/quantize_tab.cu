@@ -19,6 +19,7 @@
 //     and every warp load / store still covers whole 32-byte sectors.
 // Results are bit-identical to the reference's eager fp16 quantizer (golden vectors + oracle tests).
 #include "quantize_tab.cuh"
+#include "vcache_dev.cuh"
 #include <mutex>
 #include <string.h>
 
@@ -61,6 +62,11 @@ struct TabArgs {
     int log2Gt;               // log2(lanes per block)
     int m_lanes, log2m;       // chunks (= lanes) per micro-block
     int l2_sc_bit, nl2, l2_bytes;
+    // KV: the K / post-RoPE Q cache write; a row (b, t, h) is one block, stored at (b, h, t)
+    const uint4* rope_cos;    // fp16 [rope_rows, block] or NULL (no rotation)
+    const uint4* rope_sin;
+    const uint4* center;      // fp16 [B, H, block] or NULL: subtracted after the rotation
+    uint32_t kv_T, kv_H, rope_rows;
     TabSecond b;              // hbq_tab_mix_kernel
 };
 static_assert(sizeof(TabArgs) <= 4000, "kernel parameters are limited to 4 KB");
@@ -359,8 +365,46 @@ __device__ __forceinline__ void store_block_side(const TabArgs& a, int64_t bi, i
     }
 }
 
+// Rotary embedding and centring of the K / post-RoPE Q cache write on a thread-unit's fp16 chunks: a row is one block,
+// so chunk k's rotation partner (d +- D/2) is chunk k +- C/2 of the same thread.  Every product, the sum and the
+// difference are rounded to fp16 like the reference's tensor ops (the _rn forms keep ptxas from contracting them).
+template <int C>
+__device__ __forceinline__ void kv_rows(const TabArgs& a, uint32_t (*xb)[4], uint32_t bt, uint32_t b, uint32_t t, uint32_t h,
+                                        int Gt, int g)
+{
+    const int cpr = C * Gt;
+    if (a.rope_cos) {
+        const int64_t r0 = (int64_t)(a.rope_rows == a.kv_T ? t : bt % a.rope_rows) * cpr + g;
+        #pragma unroll
+        for (int k = 0; k < C / 2; ++k) {
+            const uint4 c0 = __ldg(a.rope_cos + r0 + k * Gt), s0 = __ldg(a.rope_sin + r0 + k * Gt);
+            const uint4 c1 = __ldg(a.rope_cos + r0 + (k + C / 2) * Gt), s1 = __ldg(a.rope_sin + r0 + (k + C / 2) * Gt);
+            const uint32_t cl[4] = {c0.x, c0.y, c0.z, c0.w}, sl[4] = {s0.x, s0.y, s0.z, s0.w};
+            const uint32_t ch[4] = {c1.x, c1.y, c1.z, c1.w}, sh[4] = {s1.x, s1.y, s1.z, s1.w};
+            #pragma unroll
+            for (int p = 0; p < 4; ++p) {
+                const uint32_t lo = xb[k][p], hi = xb[k + C / 2][p];
+                xb[k][p] = h2_bits(__hadd2_rn(__hmul2_rn(bits_h2(lo), bits_h2(cl[p])), __hmul2_rn(bits_h2(hi ^ 0x80008000u), bits_h2(sl[p]))));
+                xb[k + C / 2][p] = h2_bits(__hadd2_rn(__hmul2_rn(bits_h2(hi), bits_h2(ch[p])), __hmul2_rn(bits_h2(lo), bits_h2(sh[p]))));
+            }
+        }
+    }
+    if (a.center) {
+        const int64_t r0 = ((int64_t)b * a.kv_H + h) * cpr + g;
+        #pragma unroll
+        for (int k = 0; k < C; ++k) {
+            const uint4 cv = __ldg(a.center + r0 + k * Gt);
+            const uint32_t c[4] = {cv.x, cv.y, cv.z, cv.w};
+            #pragma unroll
+            for (int p = 0; p < 4; ++p) xb[k][p] = h2_bits(__hsub2_rn(bits_h2(xb[k][p]), bits_h2(c[p])));
+        }
+    }
+}
+
 // GT / ML: lanes per block / per micro-block as compile-time constants (0: read from the arguments).
-template <int MB, int C, int GT, int ML, bool SIDE, bool GLU>
+// KV: the K / post-RoPE Q cache write (TabArgs).  K of [4, 1999, 8 x 128] fp16: 22.0 us with the 8-byte
+// tables of quantize_lut.cu, 11.8 us here (2.8 TB/s of input and output; instruction issue bounds it).
+template <int MB, int C, int GT, int ML, bool SIDE, bool GLU, bool KV = false>
 __global__ void __launch_bounds__(TAB_THREADS, 2) hbq_tab_kernel(const TabArgs a)
 {
     extern __shared__ __align__(128) uint32_t s_tab[];
@@ -373,7 +417,10 @@ __global__ void __launch_bounds__(TAB_THREADS, 2) hbq_tab_kernel(const TabArgs a
 
     const int log2Gt = GT > 0 ? (GT == 1 ? 0 : GT == 2 ? 1 : GT == 4 ? 2 : GT == 8 ? 3 : GT == 16 ? 4 : 5) : a.log2Gt;
     const int Gt = 1 << log2Gt;
+    // warps take turns over the CTAs (not a CTA's 16 warps over consecutive units), so that a work total that is not a
+    // whole number of rounds leaves every SM the same number of warps' work
     const int64_t stride = (int64_t)gridDim.x * TAB_THREADS;
+    const int64_t u0 = ((int64_t)(tid >> 5) * gridDim.x + blockIdx.x) * 32 + lane;
 
     // raw loads of a thread-unit (zeros beyond the end)
     auto load_unit = [&](int64_t uu, uint4* rx, uint4* rg) {
@@ -390,7 +437,7 @@ __global__ void __launch_bounds__(TAB_THREADS, 2) hbq_tab_kernel(const TabArgs a
         }
     };
     #pragma unroll 1
-    for (int64_t u = (int64_t)blockIdx.x * TAB_THREADS + tid; u - lane < a.total_units; u += stride) {
+    for (int64_t u = u0; u - lane < a.total_units; u += stride) {
         const bool valid = u < a.total_units;
         const int64_t bi = u >> log2Gt;                         // block index (flat over rows)
         const int g = (int)u & (Gt - 1);                        // lane of the block
@@ -421,6 +468,14 @@ __global__ void __launch_bounds__(TAB_THREADS, 2) hbq_tab_kernel(const TabArgs a
                     xb[k][p] = h2_bits(__floats2half2_rn(__uint_as_float(xb[k][p] << 16), __uint_as_float(xb[k][p] & 0xFFFF0000u)));
         }
 
+        int64_t o0 = c0;                                        // where chunk 0 is stored
+        if (KV) {
+            const uint32_t row = valid ? (uint32_t)bi : 0u;
+            const uint32_t bt = row / a.kv_H, h = row - bt * a.kv_H, b = bt / a.kv_T, t = bt - b * a.kv_T;
+            kv_rows<C>(a, xb, bt, b, t, h, Gt, g);
+            o0 = (((int64_t)b * a.kv_H + h) * a.kv_T + t) * (C * Gt) + g;
+        }
+
         // ---- block maximum and the E5M3 shared scale (round-half-up of the 3-bit mantissa) ----
         uint32_t mx = 0u;
         #pragma unroll
@@ -447,13 +502,14 @@ __global__ void __launch_bounds__(TAB_THREADS, 2) hbq_tab_kernel(const TabArgs a
         uint32_t codes[SIDE ? C : 1], sbits[SIDE ? C : 1];
         // value * t * l1 overflows fp16 only for blocks whose maximum is within 1 % of fp16's own: one
         // warp-uniform branch between the fused form and the form that keeps each product's rounding
-        if (__all_sync(0xFFFFFFFFu, l1b < a.big_l1)) amin = unit_chunks<MB, C, ML, true, SIDE, 0>(a, dst, s_nt2, s_tabf, xb, l1b, cst, a.m_lanes, bests, codes, sbits);
-        else amin = unit_chunks<MB, C, ML, false, SIDE, 0>(a, dst, s_nt2, s_tabf, xb, l1b, cst, a.m_lanes, bests, codes, sbits);
+        constexpr int TINY = KV ? 1 : 0;                        // a second read of the inputs would rotate them again
+        if (__all_sync(0xFFFFFFFFu, l1b < a.big_l1)) amin = unit_chunks<MB, C, ML, true, SIDE, TINY>(a, dst, s_nt2, s_tabf, xb, l1b, cst, a.m_lanes, bests, codes, sbits);
+        else amin = unit_chunks<MB, C, ML, false, SIDE, TINY>(a, dst, s_nt2, s_tabf, xb, l1b, cst, a.m_lanes, bests, codes, sbits);
 
         // The reference returns +0 (not -0) when fp16(a / t) is exactly zero.  Only quotients a below 2^-19
         // can do that; deciding it needs the exact a, where the scaled division may be off: rare, so the
         // inputs are read again and the quotients redone with true divisions.
-        if (__hle2_mask(bits_h2(amin), bits_h2(0x00200020u)) != 0u && valid) {
+        if (!KV && __hle2_mask(bits_h2(amin), bits_h2(0x00200020u)) != 0u && valid) {
             const float l1f = __half2float(bits_h((uint16_t)l1b));
             #pragma unroll
             for (int k = 0; k < C; ++k) {                  // unrolled: xb must stay in registers
@@ -518,7 +574,7 @@ __global__ void __launch_bounds__(TAB_THREADS, 2) hbq_tab_kernel(const TabArgs a
                         dq[p] = *reinterpret_cast<uint32_t*>(&bb);
                     }
                 }
-                a.deq[ci] = make_uint4(dq[0], dq[1], dq[2], dq[3]);
+                a.deq[o0 + k * Gt] = make_uint4(dq[0], dq[1], dq[2], dq[3]);
             }
         }
         if (SIDE) store_block_side(a, bi, Gt, valid && g == 0, l1b, 0u, l2word);
@@ -608,9 +664,10 @@ __global__ void __launch_bounds__(MIX_THREADS, 2) hbq_tab_mix_kernel(const TabAr
     const int log2Gt = GT == 4 ? 2 : a.log2Gt;
     const int Gt = 1 << log2Gt;
     const int64_t stride = (int64_t)gridDim.x * MIX_THREADS;
+    const int64_t u0 = ((int64_t)(tid >> 5) * gridDim.x + blockIdx.x) * 32 + lane;    // as in hbq_tab_kernel
 
     #pragma unroll 1
-    for (int64_t u = (int64_t)blockIdx.x * MIX_THREADS + tid; u - lane < a.total_units; u += stride) {
+    for (int64_t u = u0; u - lane < a.total_units; u += stride) {
         const bool valid = u < a.total_units;
         const int64_t bi = u >> log2Gt;
         const int g = (int)u & (Gt - 1);
@@ -742,6 +799,117 @@ __global__ void __launch_bounds__(MIX_THREADS, 2) hbq_tab_mix_kernel(const TabAr
     }
 }
 
+
+// ---- V-cache write: blocks of 128 consecutive TOKENS per (batch, head, channel) --------------------------------
+// A CTA of 256 threads takes a tile of 128 tokens x 64 channels of [B, T, H, D], turns it through shared memory and
+// hands every channel's block to the table quantizer with the geometry of the activation kernel (four lanes a block,
+// four chunks a lane).  The tile is kept as one row of 64 token-PAIR words per channel, so that a chunk is one 16-byte
+// word: a thread of the load and store phases holds two tokens x 8 channels and regroups them with byte permutes.
+// 16-byte granules of a row are XOR-swizzled by the channel: the load phase's 8 segments x 4 words and a quarter
+// warp's 2 channels x 4 chunks each cover all 32 banks.  Tokens beyond T are the reference's zero padding.
+// Bound: instruction issue, as hbq_tab_kernel.  V of [4, 1999, 8 x 128] fp16: 28.0 us with the
+// 8-byte tables and one chunk a lane, 17.0 us here.
+constexpr int TABV_THREADS = 256, TABV_D = 64, TABV_T = 128;
+constexpr int TABV_TILE_WORDS = TABV_D * TABV_T / 2;
+
+__device__ __forceinline__ int tabv_word(int d, int tp)
+{
+    return d * (TABV_T / 2) + ((((tp >> 2) ^ ((d >> 3) & 7) ^ ((d & 1) << 2)) << 2) | (tp & 3));
+}
+
+template <int MB, int ML>
+__global__ void __launch_bounds__(TABV_THREADS, 4) hbq_tab_v_kernel(const TabArgs a, const VArgs v)
+{
+    extern __shared__ __align__(128) uint32_t s_tab[];
+    __shared__ __align__(16) uint32_t tile[TABV_TILE_WORDS];
+    __shared__ uint4 s_l1c[256];
+    __shared__ __align__(8) unsigned long long s_bar;
+    __shared__ uint32_t s_nt2[4];
+    __shared__ float s_tabf[4];
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const uint32_t dst = stage_table(a, s_tab, s_l1c, &s_bar, s_nt2, s_tabf, TABV_THREADS);
+    const int seg = tid & 7;                                     // load / store phases: 8 channels
+    #pragma unroll 1
+    for (int64_t tl = blockIdx.x; tl < v.tiles; tl += gridDim.x) {
+        const int ds = (int)(tl % v.dslabs);
+        const int64_t rest = tl / v.dslabs;
+        const int tb = (int)(rest % v.tblocks);
+        const int64_t bh = rest / v.tblocks;
+        const int64_t b = bh / v.H, h = bh - b * v.H;
+        const int64_t t0 = (int64_t)tb * TABV_T;
+        const int d0 = ds * TABV_D + seg * 8;
+        const uint16_t* src = v.in + ((b * v.T * v.H + h) * v.D + d0);
+
+        uint4 ld[4];
+        #pragma unroll
+        for (int r = 0; r < 4; ++r) {                            // tokens 2 tp, 2 tp + 1 of tp = tid / 8 and tid / 8 + 32
+            const int64_t t = t0 + 2 * ((tid >> 3) + 32 * (r >> 1)) + (r & 1);
+            ld[r] = make_uint4(0u, 0u, 0u, 0u);
+            if (t < v.T) ld[r] = __ldg(reinterpret_cast<const uint4*>(src + t * v.H * v.D));
+        }
+        #pragma unroll
+        for (int r = 0; r < 2; ++r) {
+            const int tp = (tid >> 3) + 32 * r;
+            uint32_t e[4] = {ld[2 * r].x, ld[2 * r].y, ld[2 * r].z, ld[2 * r].w};
+            uint32_t o[4] = {ld[2 * r + 1].x, ld[2 * r + 1].y, ld[2 * r + 1].z, ld[2 * r + 1].w};
+            #pragma unroll
+            for (int i = 0; i < 4; ++i) {
+                if (v.in_bf16) {
+                    e[i] = h2_bits(__floats2half2_rn(__uint_as_float(e[i] << 16), __uint_as_float(e[i] & 0xFFFF0000u)));
+                    o[i] = h2_bits(__floats2half2_rn(__uint_as_float(o[i] << 16), __uint_as_float(o[i] & 0xFFFF0000u)));
+                }
+                tile[tabv_word(seg * 8 + 2 * i, tp)] = prmt(e[i], o[i], 0x5410u);
+                tile[tabv_word(seg * 8 + 2 * i + 1, tp)] = prmt(e[i], o[i], 0x7632u);
+            }
+        }
+        __syncthreads();
+        {
+            const int d = warp * 8 + (lane >> 2), g = lane & 3;
+            uint32_t xb[4][4];
+            #pragma unroll
+            for (int k = 0; k < 4; ++k) {
+                const uint4 c = *reinterpret_cast<const uint4*>(tile + tabv_word(d, (g + 4 * k) * 4));
+                xb[k][0] = c.x; xb[k][1] = c.y; xb[k][2] = c.z; xb[k][3] = c.w;
+            }
+            const uint32_t l1b = unit_scale<4>(xb, 4, a.inv_ele_max);
+            const uint4 cst = s_l1c[l1b >> 7];
+            uint32_t bests, nocodes[1], nosigns[1];
+            if (__all_sync(0xFFFFFFFFu, l1b < a.big_l1)) unit_chunks<MB, 4, ML, true, false, 1>(a, dst, s_nt2, s_tabf, xb, l1b, cst, ML, bests, nocodes, nosigns);
+            else unit_chunks<MB, 4, ML, false, false, 1>(a, dst, s_nt2, s_tabf, xb, l1b, cst, ML, bests, nocodes, nosigns);
+            #pragma unroll
+            for (int k = 0; k < 4; ++k)
+                *reinterpret_cast<uint4*>(tile + tabv_word(d, (g + 4 * k) * 4)) = make_uint4(xb[k][0], xb[k][1], xb[k][2], xb[k][3]);
+        }
+        __syncthreads();
+        #pragma unroll
+        for (int r = 0; r < 2; ++r) {
+            const int tp = (tid >> 3) + 32 * r;
+            uint32_t w[2][4];
+            #pragma unroll
+            for (int i = 0; i < 4; ++i) {
+                const uint32_t c0 = tile[tabv_word(seg * 8 + 2 * i, tp)], c1 = tile[tabv_word(seg * 8 + 2 * i + 1, tp)];
+                w[0][i] = prmt(c0, c1, 0x5410u);
+                w[1][i] = prmt(c0, c1, 0x7632u);
+            }
+            #pragma unroll
+            for (int j = 0; j < 2; ++j) {
+                const int64_t t = t0 + 2 * tp + j;
+                if (t >= v.T) continue;
+                if (v.out_bf16) {
+                    #pragma unroll
+                    for (int i = 0; i < 4; ++i) {
+                        const float2 f = __half22float2(bits_h2(w[j][i]));
+                        const __nv_bfloat162 bb = __floats2bfloat162_rn(f.x, f.y);
+                        w[j][i] = *reinterpret_cast<const uint32_t*>(&bb);
+                    }
+                }
+                const int64_t orow = v.out_token_major ? (b * v.T + t) * v.H + h : (b * v.H + h) * v.T + t;
+                *reinterpret_cast<uint4*>(v.out + (orow * v.D + d0)) = make_uint4(w[j][0], w[j][1], w[j][2], w[j][3]);
+            }
+        }
+        __syncthreads();
+    }
+}
 
 // ---- row kernels: a per-row prologue fused in front of the quantizer --------------------------------
 // Two activation quantizers of the attention / MLP blocks consume a tensor that only exists to be quantised
@@ -1062,17 +1230,25 @@ static int table_on_device(const TabTable& t, cudaStream_t stream, const uint32_
     return HBQ_OK;
 }
 
-template <int MB, int C, int GT, int ML, bool SIDE, bool GLU>
+// CTAs for a number of thread-units: as many as are resident at once, each with at least four warps' work -- small
+// tensors are spread over the SMs (HBQ-A activations [33, 14336]: 4.8 us with 16 warps' work a CTA, 3.4 with four, 3.8
+// with two or one; [8, 4096]: 4.6, 3.1, 3.0), where staging the table costs each CTA the same.
+constexpr int TAB_MIN_WARPS = 4;
+static int tab_grid(int64_t total_units, int64_t cap)
+{
+    const int64_t need = (total_units + 32 * TAB_MIN_WARPS - 1) / (32 * TAB_MIN_WARPS);
+    return (int)(need < cap ? need : cap);
+}
+
+template <int MB, int C, int GT, int ML, bool SIDE, bool GLU, bool KV = false>
 static int launch_tab(const TabArgs& a, size_t smem, cudaStream_t stream)
 {
     int sms = 0, per_sm = 0;
     { const int rc = device_sms(&sms); if (rc) return rc; }
-    { const int rc = ensure_dynamic_smem(hbq_tab_kernel<MB, C, GT, ML, SIDE, GLU>, smem); if (rc) return rc; }
-    { const int rc = resident_ctas(hbq_tab_kernel<MB, C, GT, ML, SIDE, GLU>, TAB_THREADS, smem, &per_sm); if (rc) return rc; }
-    const int64_t need = (a.total_units + TAB_THREADS - 1) / TAB_THREADS;
-    const int64_t cap = (int64_t)sms * per_sm;
-    const int grid = (int)(need < cap ? need : cap);
-    hbq_tab_kernel<MB, C, GT, ML, SIDE, GLU><<<grid, TAB_THREADS, smem, stream>>>(a);
+    { const int rc = ensure_dynamic_smem(hbq_tab_kernel<MB, C, GT, ML, SIDE, GLU, KV>, smem); if (rc) return rc; }
+    { const int rc = resident_ctas(hbq_tab_kernel<MB, C, GT, ML, SIDE, GLU, KV>, TAB_THREADS, smem, &per_sm); if (rc) return rc; }
+    const int grid = tab_grid(a.total_units, (int64_t)sms * per_sm);
+    hbq_tab_kernel<MB, C, GT, ML, SIDE, GLU, KV><<<grid, TAB_THREADS, smem, stream>>>(a);
     HBQ_LAUNCH_CHECK("hbq_tab_kernel");
     return HBQ_OK;
 }
@@ -1092,8 +1268,7 @@ static int launch_mix(const TabArgs& a, size_t smem, cudaStream_t stream)
     { const int rc = device_sms(&sms); if (rc) return rc; }
     { const int rc = ensure_dynamic_smem(hbq_tab_mix_kernel<MB, GT, ML, SIDE>, smem); if (rc) return rc; }
     { const int rc = resident_ctas(hbq_tab_mix_kernel<MB, GT, ML, SIDE>, MIX_THREADS, smem, &per_sm); if (rc) return rc; }
-    const int64_t need = (a.total_units + MIX_THREADS - 1) / MIX_THREADS, cap = (int64_t)sms * per_sm;
-    hbq_tab_mix_kernel<MB, GT, ML, SIDE><<<(int)(need < cap ? need : cap), MIX_THREADS, smem, stream>>>(a);
+    hbq_tab_mix_kernel<MB, GT, ML, SIDE><<<tab_grid(a.total_units, (int64_t)sms * per_sm), MIX_THREADS, smem, stream>>>(a);
     HBQ_LAUNCH_CHECK("hbq_tab_mix_kernel");
     return HBQ_OK;
 }
@@ -1111,6 +1286,11 @@ static int launch_mix_geometry(const TabArgs& a, int Gt, int m, bool side, size_
 template <int MB>
 static int launch_tab_geometry(const TabArgs& a, int C, int Gt, int m, bool side, bool glu, size_t smem, cudaStream_t stream)
 {
+    if (a.kv_T) {                                            // C == 4
+        if (Gt == 4 && m == 1) return launch_tab<MB, 4, 4, 1, false, false, true>(a, smem, stream);
+        if (Gt == 4 && m == 4) return launch_tab<MB, 4, 4, 4, false, false, true>(a, smem, stream);
+        return launch_tab<MB, 4, 0, 0, false, false, true>(a, smem, stream);
+    }
     if (C == 4 && Gt == 4 && m == 1) return launch_tab_variant<MB, 4, 4, 1>(a, side, glu, smem, stream);
     if (C == 4 && Gt == 4 && m == 4) return launch_tab_variant<MB, 4, 4, 4>(a, side, glu, smem, stream);
     if (C == 4) return launch_tab_variant<MB, 4, 0, 0>(a, side, glu, smem, stream);
@@ -1237,11 +1417,14 @@ int hbq_tab_try_launch(const QArgs& q, int mb, cudaStream_t stream, bool* launch
     *launched = false;
     if (mb < 1 || mb > 2 || q.nscheme > 2 || q.nc > 4 || !q.scale_fast_e5m3) return HBQ_OK;
     if (!q.aligned || q.K != q.Kp) return HBQ_OK;
-    if (q.rope_cos || q.perm_T > 0 || q.k_center) return HBQ_OK;
+    const bool kv = q.rope_cos || q.perm_T > 0 || q.k_center;
     const bool side = q.out.codes || q.out.sign || q.out.scale_u8 || q.out.scale_h || q.out.l2_packed || q.out.l2_idx ||
                       q.out.scheme;
     const bool glu = q.glu_gate != nullptr, mix = q.nscheme == 2;
     if (!side && !q.deq) return HBQ_OK;
+    // the K / post-RoPE Q cache write: rows of one block each (the rotation partners share a thread), indices in 32 bits
+    if (kv && (mix || side || glu || q.perm_T <= 0 || q.K != q.f.block_size || q.rows > 0x7FFFFFFFll || q.rope_rows > 0x7FFFFFFFll))
+        return HBQ_OK;
     if (glu && (mix || side || q.in_bf16 || q.out_bf16)) return HBQ_OK;
     if ((reinterpret_cast<uintptr_t>(q.out.codes) & 3) || (reinterpret_cast<uintptr_t>(q.out.l2_packed) & 3) ||
         (reinterpret_cast<uintptr_t>(q.out.scale_h) & 1))
@@ -1252,7 +1435,7 @@ int hbq_tab_try_launch(const QArgs& q, int mb, cudaStream_t stream, bool* launch
     int C = 0;
     if (cpb % 4 == 0 && m <= cpb / 4) C = 4;
     else if (cpb % 2 == 0 && m <= cpb / 2) C = 2;
-    if (C == 0 || (mix && C != 4)) return HBQ_OK;
+    if (C == 0 || ((mix || kv) && C != 4)) return HBQ_OK;
     const int Gt = cpb / C;
     if (Gt > 32 || (Gt & (Gt - 1)) || (m & (m - 1))) return HBQ_OK;
 
@@ -1287,12 +1470,53 @@ int hbq_tab_try_launch(const QArgs& q, int mb, cudaStream_t stream, bool* launch
     a.l2_sc_bit = q.f.l2_sc_bit;
     a.nl2 = q.f.block_size / L;
     a.l2_bytes = (a.nl2 * a.l2_sc_bit) >> 3;
+    if (kv) {
+        a.rope_cos = reinterpret_cast<const uint4*>(q.rope_cos); a.rope_sin = reinterpret_cast<const uint4*>(q.rope_sin);
+        a.center = reinterpret_cast<const uint4*>(q.k_center);
+        a.kv_T = (uint32_t)q.perm_T; a.kv_H = (uint32_t)q.perm_H; a.rope_rows = (uint32_t)q.rope_rows;
+    }
 
     const size_t smem = (size_t)(a.entries + (mix ? a.b.entries : 0)) * 4;
     int rc;
     if (mix) rc = mb == 1 ? launch_mix_geometry<1>(a, Gt, m, side, smem, stream) : launch_mix_geometry<2>(a, Gt, m, side, smem, stream);
     else rc = mb == 1 ? launch_tab_geometry<1>(a, C, Gt, m, side, glu, smem, stream)
                       : launch_tab_geometry<2>(a, C, Gt, m, side, glu, smem, stream);
+    if (rc == HBQ_OK) *launched = true;
+    return rc;
+}
+
+template <int MB, int ML>
+static int launch_tab_v(const TabArgs& a, const VArgs& v, cudaStream_t stream)
+{
+    const size_t smem = (size_t)a.entries * 4;
+    int sms = 0, per_sm = 0;
+    { const int rc = device_sms(&sms); if (rc) return rc; }
+    { const int rc = ensure_dynamic_smem(hbq_tab_v_kernel<MB, ML>, smem); if (rc) return rc; }
+    { const int rc = resident_ctas(hbq_tab_v_kernel<MB, ML>, TABV_THREADS, smem, &per_sm); if (rc) return rc; }
+    const int64_t cap = (int64_t)sms * per_sm;
+    hbq_tab_v_kernel<MB, ML><<<(int)(v.tiles < cap ? v.tiles : cap), TABV_THREADS, smem, stream>>>(a, v);
+    HBQ_LAUNCH_CHECK("hbq_tab_v_kernel");
+    return HBQ_OK;
+}
+
+int hbq_tab_v_try_launch(const QArgs& q, int mb, const void* in, void* out, int in_bf16, int out_bf16, int64_t B, int64_t T,
+                         int64_t H, int64_t D, int out_token_major, cudaStream_t stream, bool* launched)
+{
+    *launched = false;
+    const int L = q.f.l2_block_size;
+    if (mb < 1 || mb > 2 || q.nscheme != 1 || q.nc > 4 || !q.scale_fast_e5m3) return HBQ_OK;
+    if (q.f.block_size != TABV_T || (L != 8 && L != 32) || ((reinterpret_cast<uintptr_t>(in) | reinterpret_cast<uintptr_t>(out)) & 15))
+        return HBQ_OK;
+    VArgs v;
+    if (!v_args_fill(&v, in, out, in_bf16, out_bf16, B, T, H, D, q.f.block_size, out_token_major) || v.tiles == 0) return HBQ_OK;
+    TabArgs a;
+    bool ok = false;
+    { const int rc = fill_format(q, mb, stream, &a, &ok); if (rc) return rc; }
+    if (!ok) return HBQ_OK;
+    a.m_lanes = L / 8;
+    int rc;
+    if (mb == 1) rc = L == 8 ? launch_tab_v<1, 1>(a, v, stream) : launch_tab_v<1, 4>(a, v, stream);
+    else rc = L == 8 ? launch_tab_v<2, 1>(a, v, stream) : launch_tab_v<2, 4>(a, v, stream);
     if (rc == HBQ_OK) *launched = true;
     return rc;
 }

@@ -18,4 +18,8 @@ bool hbq_tab_table(int mb, const float* tab, int nc, TabTable* out);
 // Runs the byte-table kernel if the (validated) HBQ arguments fit it; *launched tells whether it did.
 int hbq_tab_try_launch(const QArgs& qa, int mb, cudaStream_t stream, bool* launched);
 
+// The token-axis (V-cache) write in blocks of 128 tokens; the other block sizes and formats are hbq_lut_v_launch's.
+int hbq_tab_v_try_launch(const QArgs& qa, int mb, const void* in, void* out, int in_bf16, int out_bf16, int64_t B, int64_t T,
+                         int64_t H, int64_t D, int out_token_major, cudaStream_t stream, bool* launched);
+
 }  // namespace hbq
