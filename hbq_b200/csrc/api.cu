@@ -84,6 +84,10 @@ int transpose_launch(const void*, void*, int64_t, int64_t, cudaStream_t);
 int gemm_tc_status(int*);
 int gemm_tc_status_reset();
 int gemm_tc_reserve_sms(int n);
+int gemm_tc_grouped_launch(const void*, int64_t, const int*, int, const void* const*, void* const*, const int*, int64_t, int64_t, int,
+                           int, int, cudaStream_t);
+int moe_route_launch(const int64_t*, int64_t, int, int, int*, int64_t*, int*, cudaStream_t);                      // moe.cu
+int moe_combine_launch(const void*, const void*, const int*, int64_t, int, int64_t, void*, cudaStream_t);
 int64_t gemm_w4_prepacked_bytes(int64_t, int64_t, int);
 int gemm_w4_prepack(const hbq_packed_out*, int64_t, int64_t, const hbq_format*, int, void*, cudaStream_t);
 int64_t gemm_w4_workspace_bytes(int64_t, int64_t, int64_t);
@@ -256,6 +260,34 @@ int hbq_gemm_wait_selftest(const void* A, const void* W, void* C, int64_t M, int
     if ((((uintptr_t)A | (uintptr_t)W | (uintptr_t)C) & 15) || !gemm_tc_eligible(M, N, K, mode, group_k, group_n))
         return HBQ_ERR_UNSUPPORTED;
     return gemm_tc_launch_ex(A, W, C, M, N, K, mode, group_k, group_n, nullptr, (cudaStream_t)stream, poll_limit, 1);
+}
+
+int hbq_moe_route(const int64_t* ids, int64_t tokens, int top_k, int experts, int32_t* offsets, int64_t* src_rows,
+                  int32_t* pos, void* stream)
+{
+    return moe_route_launch(ids, tokens, top_k, experts, offsets, src_rows, pos, (cudaStream_t)stream);
+}
+
+int hbq_gemm_grouped(const void* A, int64_t rows, const int32_t* offsets, int entries, const void* const* W_host,
+                     void* const* C_host, const int32_t* expert_host, int64_t N, int64_t K, int mode, int group_k,
+                     int group_n, void* stream)
+{
+    if (rows < 0 || N < 0 || K < 0 || entries < 0) return HBQ_ERR_ARG;
+    if (rows == 0 || N == 0 || entries == 0) return HBQ_OK;
+    if (!offsets || !W_host || !C_host || !expert_host) return HBQ_ERR_ARG;
+    for (int i = 0; i < entries; ++i) {
+        const int rc = check_gemm_args(A, W_host[i], C_host[i], rows, N, K, mode, group_k, group_n);
+        if (rc) return rc;
+        if (expert_host[i] < 0) return HBQ_ERR_ARG;
+    }
+    return gemm_tc_grouped_launch(A, rows, offsets, entries, W_host, C_host, expert_host, N, K, mode, group_k, group_n,
+                                  (cudaStream_t)stream);
+}
+
+int hbq_moe_combine(const void* y_rows, const void* weights, const int32_t* pos, int64_t tokens, int top_k, int64_t hidden,
+                    void* out, void* stream)
+{
+    return moe_combine_launch(y_rows, weights, pos, tokens, top_k, hidden, out, (cudaStream_t)stream);
 }
 
 int64_t hbq_gemm_w4_prepacked_bytes(int64_t N, int64_t K, int container_bits)

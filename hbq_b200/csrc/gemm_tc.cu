@@ -28,6 +28,7 @@
 #include <math.h>
 #include <atomic>
 #include <mutex>
+#include <string.h>
 
 namespace hbq {
 
@@ -138,11 +139,55 @@ struct TcArgs {
 };
 constexpr uint32_t kDefaultPollLimit = 1u << 23;
 
+// One output tile: where its operands start, which rows it may store and where.
+struct TcTile {
+    const CUtensorMap* mapB;
+    __half* C;
+    int m0, n0, row_end;
+};
+
+// Tile order of one product: m fastest, so that CTAs that run together share a W tile.
+struct PlainTiles {
+    const CUtensorMap* mapB;
+    const TcArgs& args;
+    int bn;
+    __device__ __forceinline__ int total() const { return args.tiles_m * args.tiles_n; }
+    __device__ __forceinline__ TcTile tile(int t) const
+    {
+        return {mapB, args.C, (t % args.tiles_m) * BM, (t / args.tiles_m) * bn, args.M};
+    }
+};
+
+// Several products over row segments of one A (the experts of a sparse MoE block): entry i multiplies rows
+// [off[expert], off[expert + 1]) by its own W into its own C.  The row offsets are read on the device.
+constexpr int TC_MAX_ENTRIES = 16;
+struct GroupArgs {
+    CUtensorMap mapB[TC_MAX_ENTRIES];
+    __half* C[TC_MAX_ENTRIES];
+    int expert[TC_MAX_ENTRIES];
+    const int* offsets;
+    int entries;
+};
+struct GroupTiles {
+    const GroupArgs& g;
+    const TcArgs& args;
+    const int* first;           // shared memory: first tile of each entry, then the total
+    const int* rows;            // first and last + 1 row of each entry
+    int bn;
+    __device__ __forceinline__ int total() const { return first[g.entries]; }
+    __device__ __forceinline__ TcTile tile(int t) const
+    {
+        int e = 0;
+        while (e + 1 < g.entries && t >= first[e + 1]) ++e;
+        const int r0 = rows[2 * e], r1 = rows[2 * e + 1];
+        const int tiles_m = (r1 - r0 + BM - 1) / BM, u = t - first[e];
+        return {&g.mapB[e], g.C[e], r0 + (u % tiles_m) * BM, (u / tiles_m) * bn, r1};
+    }
+};
+
 // ---- the kernel ------------------------------------------------------------------------------
-template <int MODE, int GN, int BN, int NSTAGE>
-__global__ void __launch_bounds__(NTHREADS, 1)
-gemm_tc_kernel(const __grid_constant__ CUtensorMap mapA, const __grid_constant__ CUtensorMap mapB,
-               const TcArgs args)
+template <int MODE, int GN, int BN, int NSTAGE, class Tiles>
+__device__ __forceinline__ void gemm_tc_body(const CUtensorMap& mapA, const Tiles& sched, const TcArgs& args)
 {
     constexpr int STAGE_BYTES = A_BYTES + BN * BK * 2;
     // kind::f16: D fp32, A/B fp16, both K-major, M = 128, N = BN
@@ -178,7 +223,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap mapA, const __grid_constant__
     tc_fence_after();
     const uint32_t tmem_base = *tmem_base_smem;
 
-    const int total_tiles = args.tiles_m * args.tiles_n;
+    const int total_tiles = sched.total();
     const int total_k16 = args.k_stages * (BK / 16);
 
     // Register re-balancing between the warpgroups: the control warpgroup (warps 0-3) gives registers
@@ -191,13 +236,13 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap mapA, const __grid_constant__
             uint32_t stage = 0, phase = 0;
             bool ok = true;
             for (int t = blockIdx.x; t < total_tiles && ok && !args.withhold_loads; t += gridDim.x) {
-                const int m0 = (t % args.tiles_m) * BM, n0 = (t / args.tiles_m) * BN;
+                const TcTile tl = sched.tile(t);
                 for (int ks = 0; ks < args.k_stages; ++ks) {
                     if (!(ok = mbar_wait(bar_empty + 8 * stage, phase ^ 1u, abort_flag, 1, args.poll_limit))) break;
                     const uint32_t sa = tiles + stage * STAGE_BYTES, sb = sa + A_BYTES;
                     mbar_expect_tx(bar_full + 8 * stage, STAGE_BYTES);
-                    tma_load_2d(sa, &mapA, ks * BK, m0, bar_full + 8 * stage);
-                    tma_load_2d(sb, &mapB, ks * BK, n0, bar_full + 8 * stage);
+                    tma_load_2d(sa, &mapA, ks * BK, tl.m0, bar_full + 8 * stage);
+                    tma_load_2d(sb, tl.mapB, ks * BK, tl.n0, bar_full + 8 * stage);
                     if (++stage == NSTAGE) { stage = 0; phase ^= 1u; }
                 }
             }
@@ -305,7 +350,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap mapA, const __grid_constant__
         uint32_t chunk = 0;
         bool ok = true;
         for (int t = blockIdx.x; t < total_tiles && ok; t += gridDim.x) {
-            const int m0 = (t % args.tiles_m) * BM, n0 = (t / args.tiles_m) * BN;
+            const TcTile tl = sched.tile(t);
             __half2 acc[EPI_COLS / 2];
             #pragma unroll
             for (int i = 0; i < EPI_COLS / 2; ++i) acc[i] = __float2half2_rn(0.f);
@@ -339,10 +384,10 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap mapA, const __grid_constant__
             }
             if (!ok) break;
             // ---- write the thread's row: EPI_COLS columns starting at n0 + cgrp*EPI_COLS ----
-            const int row = m0 + quarter * 32 + lane;
-            const int col0 = n0 + cgrp * EPI_COLS;
-            if (row < args.M) {
-                __half* cp = args.C + (int64_t)row * args.N + col0;
+            const int row = tl.m0 + quarter * 32 + lane;
+            const int col0 = tl.n0 + cgrp * EPI_COLS;
+            if (row < tl.row_end) {
+                __half* cp = tl.C + (int64_t)row * args.N + col0;
                 #pragma unroll
                 for (int g = 0; g < EPI_COLS / 8; ++g) {
                     const int col = col0 + g * 8;
@@ -373,6 +418,43 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap mapA, const __grid_constant__
         tc_fence_after();
         asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, 512;" ::"r"(tmem_base) : "memory");
     }
+}
+
+
+template <int MODE, int GN, int BN, int NSTAGE>
+__global__ void __launch_bounds__(NTHREADS, 1)
+gemm_tc_kernel(const __grid_constant__ CUtensorMap mapA, const __grid_constant__ CUtensorMap mapB,
+               const __grid_constant__ TcArgs args)
+{
+    const PlainTiles sched = {&mapB, args, BN};
+    gemm_tc_body<MODE, GN, BN, NSTAGE>(mapA, sched, args);
+}
+
+// All experts' products of one projection (or of two that share their input) in one launch.  One launch per expert
+// leaves SMs idle at the end of each (250 rows x [4096, 14336]: 64 tiles of 128 columns on 148 SMs) and needs the row
+// counts on the host.  1000 tokens, top-2 of 8 experts of 4096 x 14336, fp32 accumulation: the 24 products 1368 us, the two
+// launches (w1 and w3 together, w2) 806 us; tiles of 128 columns instead of 256: 628 + 334 us against 537 + 304.  Bound:
+// the tensor pipe at 1.1 PFLOP/s of the padded rows, with W streaming from HBM at 3.5 TB/s beside it.
+template <int MODE, int GN, int BN, int NSTAGE>
+__global__ void __launch_bounds__(NTHREADS, 1)
+gemm_tc_grouped_kernel(const __grid_constant__ CUtensorMap mapA, const __grid_constant__ GroupArgs group,
+                       const __grid_constant__ TcArgs args)
+{
+    __shared__ int s_first[TC_MAX_ENTRIES + 1], s_rows[2 * TC_MAX_ENTRIES];
+    if (threadIdx.x == 0) {
+        int n = 0;
+        for (int e = 0; e < group.entries; ++e) {
+            const int r0 = __ldg(group.offsets + group.expert[e]), r1 = __ldg(group.offsets + group.expert[e] + 1);
+            s_first[e] = n;
+            s_rows[2 * e] = r0;
+            s_rows[2 * e + 1] = r1;
+            n += (r1 - r0 + BM - 1) / BM * args.tiles_n;
+        }
+        s_first[group.entries] = n;
+    }
+    __syncthreads();
+    const GroupTiles sched = {group, args, s_first, s_rows, BN};
+    gemm_tc_body<MODE, GN, BN, NSTAGE>(mapA, sched, args);
 }
 
 
@@ -552,6 +634,68 @@ int gemm_tc_launch(const void* A, const void* W, void* C, int64_t M, int64_t N, 
                    int group_k, int group_n, const void* bias, cudaStream_t stream)
 {
     return gemm_tc_launch_ex(A, W, C, M, N, K, mode, group_k, group_n, bias, stream, 0, 0);
+}
+
+template <int MODE, int GN>
+static int launch_grouped(const CUtensorMap& ma, const GroupArgs& g, const TcArgs& args, int grid, cudaStream_t stream)
+{
+    if (args.bn == 128) {
+        { const int rc = ensure_dynamic_smem(gemm_tc_grouped_kernel<MODE, GN, 128, 6>, smem_bytes(128, 6)); if (rc) return rc; }
+        gemm_tc_grouped_kernel<MODE, GN, 128, 6><<<grid, NTHREADS, smem_bytes(128, 6), stream>>>(ma, g, args);
+    } else {
+        { const int rc = ensure_dynamic_smem(gemm_tc_grouped_kernel<MODE, GN, 256, 4>, smem_bytes(256, 4)); if (rc) return rc; }
+        gemm_tc_grouped_kernel<MODE, GN, 256, 4><<<grid, NTHREADS, smem_bytes(256, 4), stream>>>(ma, g, args);
+    }
+    HBQ_LAUNCH_CHECK("gemm_tc_grouped_kernel");
+    return HBQ_OK;
+}
+
+// A [rows, K]; entry i: C[i][r, :] = A[r, :] * W[i][N, K]^T for the rows offsets[expert[i]] .. offsets[expert[i] + 1] - 1
+// (device int32, ascending, at most `rows`).  Launches of up to TC_MAX_ENTRIES entries.
+int gemm_tc_grouped_launch(const void* A, int64_t rows, const int* offsets, int entries, const void* const* W, void* const* C,
+                           const int* expert, int64_t N, int64_t K, int mode, int group_k, int group_n, cudaStream_t stream)
+{
+    if (!gemm_tc_eligible(rows, N, K, mode, group_k, group_n)) return HBQ_ERR_UNSUPPORTED;
+    if (mode == HBQ_ACC_PSUM_E3M4 || (mode == HBQ_ACC_PSUM_INT8 && group_n != 32)) return HBQ_ERR_UNSUPPORTED;
+    uintptr_t bits = reinterpret_cast<uintptr_t>(A);
+    for (int i = 0; i < entries; ++i) bits |= reinterpret_cast<uintptr_t>(W[i]) | reinterpret_cast<uintptr_t>(C[i]);
+    if (bits & 15) return HBQ_ERR_ALIGN;
+    int sms = 0;
+    { const int rc = device_sms(&sms); if (rc) return rc; }
+    CUtensorMap ma;
+    { const int rc = make_map(&ma, A, rows, K, BM); if (rc) return rc; }
+    TcArgs args;
+    memset(&args, 0, sizeof(args));
+    args.M = (int)rows; args.N = (int)N; args.K = (int)K;
+    // 128-column tiles, as for one product, where even one row tile per entry and the rows' own tiles of 256 columns
+    // would leave more than half of the SMs without work
+    const int64_t tiles256 = ((rows < entries ? rows : entries) + rows / BM) * ((N + 255) / 256);
+    args.bn = (N <= 128 || tiles256 * 2 <= sms) ? 128 : 256;
+    args.tiles_n = (int)((N + args.bn - 1) / args.bn);
+    args.k_stages = (int)((K + BK - 1) / BK);
+    args.chunk_k16 = (mode == HBQ_ACC_FP32) ? args.k_stages * (BK / 16) : group_k / 16;
+    args.issuers = 2;
+    args.poll_limit = kDefaultPollLimit;
+    const int usable = sms - g_reserved_sms.load() > 0 ? sms - g_reserved_sms.load() : 1;
+    for (int e0 = 0; e0 < entries; e0 += TC_MAX_ENTRIES) {
+        GroupArgs g;
+        memset(&g, 0, sizeof(g));
+        g.offsets = offsets;
+        g.entries = entries - e0 < TC_MAX_ENTRIES ? entries - e0 : TC_MAX_ENTRIES;
+        for (int i = 0; i < g.entries; ++i) {
+            { const int rc = make_map(&g.mapB[i], W[e0 + i], N, K, args.bn); if (rc) return rc; }
+            g.C[i] = (__half*)C[e0 + i];
+            g.expert[i] = expert[e0 + i];
+        }
+        int rc;
+        switch (mode) {
+            case HBQ_ACC_FP32: rc = launch_grouped<HBQ_ACC_FP32, 32>(ma, g, args, usable, stream); break;
+            case HBQ_ACC_GROUPED: rc = launch_grouped<HBQ_ACC_GROUPED, 32>(ma, g, args, usable, stream); break;
+            default: rc = launch_grouped<HBQ_ACC_PSUM_INT8, 32>(ma, g, args, usable, stream); break;
+        }
+        if (rc) return rc;
+    }
+    return HBQ_OK;
 }
 
 int gemm_tc_reserve_sms(int n)

@@ -15,7 +15,9 @@ router is replicated.  Per call:
 3. each rank runs its experts on the rows it received: ``w2(aq2(silu(w1(x)) * w3(x)))``;
 4. the results travel back (fp16), are weighted by the router and summed per token.
 
-With one rank (or no process group) every expert is local and no collective runs.
+With one rank (or no process group) every expert is local and no collective runs; where the experts agree in shape,
+formats and accumulation model they run as grouped products over row offsets that stay on the device (``hbq_moe_route``,
+``hbq_gemm_grouped``, ``hbq_moe_combine``), so that the call reads nothing back.
 """
 from __future__ import annotations
 
@@ -26,9 +28,12 @@ import torch.distributed as dist
 import torch.nn as nn
 import torch.nn.functional as F
 
+from . import _lib
+from .gemm import gemm_grouped
 from .kvcache import swiglu_quantize
 from .module import QLinear
-from .quantizer import PackedTensor, _QBase, dequantize_packed
+from .ops import FP16AccumMatMul, FP32AccumMatMul
+from .quantizer import PackedTensor, _CudaBlockQuantizer, _ptr, _QBase, _stream_ptr, dequantize_packed
 
 
 def _world(group) -> int:
@@ -37,6 +42,22 @@ def _world(group) -> int:
 
 def _rank(group) -> int:
     return dist.get_rank(group) if dist.is_available() and dist.is_initialized() else 0
+
+
+def _hooked(m: nn.Module) -> bool:
+    return bool(m._forward_hooks or m._forward_pre_hooks or "forward" in m.__dict__ or nn.modules.module._has_any_global_hook())
+
+
+def _accumulation(ops):
+    """``(mode, group_k, group_n)`` of a linear layer's accumulation operator where the grouped GEMM has that model."""
+    if type(ops) is FP32AccumMatMul and not _hooked(ops):
+        return _lib.ACC_FP32, 0, 0
+    if type(ops) is FP16AccumMatMul and not _hooked(ops) and ops.group_size in (64, 128):
+        if ops.quant_block_size is None:
+            return _lib.ACC_GROUPED, ops.group_size, 0
+        if ops.quant_block_size == 32:
+            return _lib.ACC_PSUM_INT8, ops.group_size, 32
+    return None
 
 
 class QuantExpert(nn.Module):
@@ -121,6 +142,75 @@ class ExpertParallelMoE(nn.Module):
                                shaped.get("sign"), shaped.get("scale_u8"), shaped.get("l2_packed"), shaped.get("scheme"))
         return dequantize_packed(arrived)
 
+    # ---- every expert on this GPU: no host read ------------------------------------------------------
+    def _grouped_model(self):
+        """``(mode, group_k, group_n)`` of the grouped GEMM when the local experts can run as two grouped products
+        around one activation / quantizer pass, else None: one rank, plain ``QuantExpert`` layers (nothing between
+        or around their linear layers: hooks, biases, output quantizers, the non-finite guard) on fp16 CUDA weights of
+        one shape, one accumulation model and one ``w2`` input quantizer, and no gradient to record."""
+        if self.world != 1 or torch.is_grad_enabled() or not 0 < self.num_experts <= 256:
+            return None
+        ex0 = self.experts[0]
+        model = _accumulation(ex0.w1.ops)
+        if model is None or not isinstance(ex0.w2.aq, _CudaBlockQuantizer) or getattr(ex0.w2.aq, "keep_l2_scale", False):
+            return None
+        fmt = ex0.w2.aq._format()
+        key = [getattr(fmt, n) for n, _ in fmt._fields_]
+        if fmt.per_tensor_scale:                                       # one maximum per expert's tensor
+            return None
+        dev = ex0.w1.weight.device
+        if dev.type != "cuda" or self.hidden % 8 or self.inter % 8:
+            return None
+        for ex in self.experts:
+            if type(ex) is not QuantExpert or _hooked(ex) or type(ex.w2.aq) is not type(ex0.w2.aq) or ex.w2.aq.out_dtype is not None or \
+                    _hooked(ex.w2.aq):
+                return None
+            f = ex.w2.aq._format()
+            if [getattr(f, n) for n, _ in f._fields_] != key:
+                return None
+            for lin, shape in ((ex.w1, (self.inter, self.hidden)), (ex.w3, (self.inter, self.hidden)), (ex.w2, (self.hidden, self.inter))):
+                w = lin.weight
+                if (type(lin) is not QLinear or _hooked(lin) or lin.bias is not None or lin.check_finite or lin.w4_weight is not None
+                        or type(lin.yq) is not _QBase or _hooked(lin.yq) or _accumulation(lin.ops) != model
+                        or w.dtype != torch.float16 or w.device != dev or tuple(w.shape) != shape or not w.is_contiguous()
+                        or w.data_ptr() % 16):
+                    return None
+                if lin is not ex.w2 and (type(lin.aq) is not _QBase or _hooked(lin.aq)):
+                    return None
+        return model
+
+    def _begin_local(self, lead, x2d, w, idx) -> dict:
+        T, dev = x2d.shape[0], x2d.device
+        idx = idx.contiguous()
+        i32 = dict(dtype=torch.int32, device=dev)
+        offsets, pos = torch.empty(self.num_experts + 1, **i32), torch.empty(T * self.top_k, **i32)
+        src_rows = torch.empty(T * self.top_k, dtype=torch.int64, device=dev)
+        with _lib.device_guard(dev):
+            rc = _lib.lib().hbq_moe_route(_ptr(idx), T, self.top_k, self.num_experts, _ptr(offsets), _ptr(src_rows), _ptr(pos),
+                                          _stream_ptr(dev))
+        _lib.check(rc, "hbq_moe_route")
+        return dict(lead=lead, x2d=x2d, w=w, offsets=offsets, src_rows=src_rows, pos=pos)
+
+    def _finish_local(self, st: dict) -> torch.Tensor:
+        x2d = st["x2d"]
+        T, dev = x2d.shape[0], x2d.device
+        mode, group_k, group_n = st["model"]
+        xq = self._dispatch(x2d, st["src_rows"], None, None)
+        n, E = xq.shape[0], self.num_experts
+        a, b = (torch.empty((n, self.inter), dtype=torch.float16, device=dev) for _ in range(2))
+        gemm_grouped(xq, st["offsets"], [ex.w1.weight for ex in self.experts] + [ex.w3.weight for ex in self.experts],
+                     [a] * E + [b] * E, list(range(E)) * 2, mode, group_k, group_n)
+        h = swiglu_quantize(a, b, self.experts[0].w2.aq)
+        y_rows = torch.empty((n, self.hidden), dtype=torch.float16, device=dev)
+        gemm_grouped(h, st["offsets"], [ex.w2.weight for ex in self.experts], [y_rows] * E, range(E), mode, group_k, group_n)
+        w = st["w"].contiguous()
+        y = torch.empty((T, self.hidden), dtype=torch.float16, device=dev)
+        with _lib.device_guard(dev):
+            rc = _lib.lib().hbq_moe_combine(_ptr(y_rows), _ptr(w), _ptr(st["pos"]), T, self.top_k, self.hidden, _ptr(y),
+                                            _stream_ptr(dev))
+        _lib.check(rc, "hbq_moe_combine")
+        return y.reshape(*st["lead"], self.hidden)
+
     # ---- forward ---------------------------------------------------------------------------------
     # The block needs one host read (the per-rank row counts size the all-to-all).  It is split in two so that a caller
     # with several independent batches can put other launches between the exchange of the counts and the read:
@@ -130,6 +220,9 @@ class ExpertParallelMoE(nn.Module):
         lead = x.shape[:-1]
         x2d = x.reshape(-1, self.hidden)
         w, idx = self.route(x2d)
+        model = self._grouped_model() if x2d.is_cuda and x2d.dtype == torch.float16 and x2d.shape[0] else None
+        if model is not None:
+            return dict(self._begin_local(lead, x2d, w, idx), model=model)
         flat_e = idx.reshape(-1)                                       # expert of copy c = (token c // k, choice c % k)
         order = torch.sort(flat_e, stable=True).indices               # copies grouped by expert, hence by rank
         src_rows = torch.div(order, self.top_k, rounding_mode="floor")
@@ -153,6 +246,8 @@ class ExpertParallelMoE(nn.Module):
         return st
 
     def finish(self, st: dict) -> torch.Tensor:
+        if "model" in st:
+            return self._finish_local(st)
         lead, x2d, w, order, src_rows = st["lead"], st["x2d"], st["w"], st["order"], st["src_rows"]
         T = x2d.shape[0]
         if st["event"] is not None:

@@ -3,7 +3,7 @@
 from __future__ import annotations
 
 import ctypes
-from typing import Optional
+from typing import Optional, Sequence
 
 import torch
 
@@ -54,6 +54,25 @@ def gemm(a: torch.Tensor, b: torch.Tensor, mode: int, group_k: int = 0, group_n:
                             _ptr(bias), _ptr(ws), ws_bytes, stream)
     _lib.check(rc, "hbq_gemm")
     return c
+
+
+def gemm_grouped(a: torch.Tensor, offsets: torch.Tensor, weights: Sequence[torch.Tensor], outs: Sequence[torch.Tensor],
+                 experts: Sequence[int], mode: int, group_k: int = 0, group_n: int = 0) -> None:
+    """``hbq_gemm_grouped``: ``outs[i][r] = a[r] @ weights[i].T`` for the rows of expert ``experts[i]``, i.e.
+    ``offsets[e] .. offsets[e + 1] - 1`` (int32 on the device, read there).  Every weight is a contiguous fp16 [N, K]
+    tensor and every output a contiguous fp16 [rows, N] tensor on ``a``'s device."""
+    rows, K = a.shape
+    N = weights[0].shape[0]
+    for t, shape in [(a, (rows, K))] + [(w, (N, K)) for w in weights] + [(c, (rows, N)) for c in outs]:
+        if t.dtype != torch.float16 or tuple(t.shape) != shape or t.device != a.device or not t.is_contiguous():
+            raise RuntimeError("gemm_grouped takes contiguous fp16 tensors of matching shapes on one device")
+    n = len(weights)
+    vp = ctypes.c_void_p * n
+    with _lib.device_guard(a.device):
+        rc = _lib.lib().hbq_gemm_grouped(_ptr(a), rows, _ptr(offsets), n, vp(*[w.data_ptr() for w in weights]),
+                                         vp(*[c.data_ptr() for c in outs]), (ctypes.c_int32 * n)(*experts), N, K, mode,
+                                         group_k, group_n, _stream_ptr(a.device))
+    _lib.check(rc, "hbq_gemm_grouped")
 
 
 def gemm_status() -> int:

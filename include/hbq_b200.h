@@ -236,6 +236,22 @@ int hbq_gemm_wait_selftest(const void* A, const void* W, void* C, int64_t M, int
 
 /* ---- GEMM on the packed weight (decode shapes) ---------------------------------------------- */
 
+/* Sparse MoE block with every expert on this GPU (the routing, the expert layers and the weighted sum of the
+ * MixtralSparseMoeBlock whose experts the reference patches, src/module.py:597-622), without a host read.
+ *   hbq_moe_route    ids [tokens, top_k] (int64 expert of each copy) -> offsets [experts + 1], src_rows [tokens * top_k]
+ *                    (token of each copy, copies stably sorted by expert), pos [tokens * top_k] (a copy's sorted row).
+ *   hbq_gemm_grouped entry i: C_host[i][r, :] = A[r, :] * W_host[i][N, K]^T for the rows of expert expert_host[i], i.e.
+ *                    offsets[e] .. offsets[e + 1] - 1; A [rows, K], accumulation model as hbq_gemm (FP32, GROUPED,
+ *                    PSUM_INT8 with group_n = 32).  W_host / C_host / expert_host are host arrays of `entries`.
+ *   hbq_moe_combine  out[t, :] = sum_j fp16(y_rows[pos[t * top_k + j], :] * weights[t, j]). */
+int hbq_moe_route(const int64_t* ids, int64_t tokens, int top_k, int experts, int32_t* offsets, int64_t* src_rows,
+                  int32_t* pos, void* stream);
+int hbq_gemm_grouped(const void* A, int64_t rows, const int32_t* offsets, int entries, const void* const* W_host,
+                     void* const* C_host, const int32_t* expert_host, int64_t N, int64_t K, int mode, int group_k,
+                     int group_n, void* stream);
+int hbq_moe_combine(const void* y_rows, const void* weights, const int32_t* pos, int64_t tokens, int top_k, int64_t hidden,
+                    void* out, void* stream);
+
 /* C[M,N] = X[M,K] * deq(W)[N,K]^T for M <= 128 tokens, reading W as packed 4-bit codes, block scales and
  * micro-scale indices (0.5625 B per weight) and expanding it to the fp16 fake-quantised values on chip (tensor memory)
  * in front of the tensor core; fp32 accumulation, fp16 output, bias as in hbq_gemm.  Replaces, for a statically
