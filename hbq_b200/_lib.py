@@ -5,10 +5,13 @@ There is no fallback: if the shared object is missing, or a call fails, an excep
 from __future__ import annotations
 
 import ctypes
+import importlib.machinery
+import importlib.util
 import os
 
 HERE = os.path.dirname(os.path.abspath(__file__))
 LIB_PATH = os.path.join(HERE, "lib", "libhbq_b200.so")
+HOST_PATH = os.path.join(HERE, "lib", "hbq_host.so")
 
 KIND_MXFP, KIND_MXINT, KIND_HBQ, KIND_MXEX, KIND_VSQ = 0, 1, 2, 3, 4
 ERR_UNSUPPORTED = -2          # HBQ_ERR_UNSUPPORTED
@@ -97,6 +100,27 @@ def lib() -> ctypes.CDLL:
     L.hbq_launch_count.restype = i64
     _lib = L
     return L
+
+
+_host = None
+
+
+def host():
+    """The torch-facing module of the hot entry points (``csrc/host.cpp``), bound to this process's library."""
+    global _host
+    if _host is not None:
+        return _host
+    L = lib()
+    if not os.path.exists(HOST_PATH):
+        raise HbqError(f"{HOST_PATH} is missing: build it with `python -m hbq_b200.build`")
+    import torch  # noqa: F401  (the module links against torch's libraries, which this loads)
+    loader = importlib.machinery.ExtensionFileLoader("hbq_host", HOST_PATH)
+    m = importlib.util.module_from_spec(importlib.util.spec_from_loader("hbq_host", loader))
+    loader.exec_module(m)
+    m.bind(*(ctypes.cast(f, ctypes.c_void_p).value for f in (L.hbq_quantize, L.hbq_gemm, L.hbq_gemm_workspace_bytes,
+                                                             L.hbq_gemm_w4)))
+    _host = m
+    return m
 
 
 class _NoGuard:

@@ -1,7 +1,8 @@
-"""Build step: compile the CUDA sources under ``csrc/`` into ``lib/libhbq_b200.so``.
+"""Build step: compile the CUDA sources under ``csrc/`` into ``lib/libhbq_b200.so`` and the
+torch-facing entry points (``csrc/host.cpp``) into ``lib/hbq_host.so``.
 
 The library targets sm_100a only and depends on nothing but the CUDA runtime, so it
-cross-compiles on a machine without a GPU::
+cross-compiles on a machine without a GPU; the module is built against the installed torch::
 
     python -m hbq_b200.build
 """
@@ -11,11 +12,14 @@ import os
 import shutil
 import subprocess
 import sys
+import sysconfig
 
 HERE = os.path.dirname(os.path.abspath(__file__))
 CSRC = os.path.join(HERE, "csrc")
 LIB_DIR = os.path.join(HERE, "lib")
 LIB_PATH = os.path.join(LIB_DIR, "libhbq_b200.so")
+HOST_PATH = os.path.join(LIB_DIR, "hbq_host.so")
+HOST_SOURCE = os.path.join(CSRC, "host.cpp")
 SOURCES = ["api.cu", "quantize.cu", "quantize_lut.cu", "quantize_tab.cu", "quantize_extra.cu", "dequantize.cu", "gemm_simt.cu", "gemm_tc.cu", "gemm_packed.cu", "gemm_static.cu", "moe.cu"]
 HEADERS = [os.path.join(CSRC, "common.cuh"), os.path.join(CSRC, "quantize_dev.cuh"), os.path.join(CSRC, "vcache_dev.cuh"), os.path.join(CSRC, "quantize_tab.cuh"), os.path.join(CSRC, "tc_dev.cuh"), os.path.join(HERE, "..", "include", "hbq_b200.h")]
 NVCC_FLAGS = ["-gencode", "arch=compute_100a,code=sm_100a", "-lineinfo", "-O3", "-std=c++17",
@@ -29,19 +33,41 @@ def _nvcc() -> str:
     raise RuntimeError("nvcc not found; it is needed to build libhbq_b200.so")
 
 
+def _older(path: str, deps) -> bool:
+    return not os.path.exists(path) or any(os.path.getmtime(d) > os.path.getmtime(path) for d in deps)
+
+
 def is_stale() -> bool:
-    if not os.path.exists(LIB_PATH):
-        return True
-    t = os.path.getmtime(LIB_PATH)
-    deps = [os.path.join(CSRC, s) for s in SOURCES] + HEADERS
-    return any(os.path.getmtime(d) > t for d in deps)
+    return _older(LIB_PATH, [os.path.join(CSRC, s) for s in SOURCES] + HEADERS)
+
+
+def _host_command():
+    import torch
+    root = os.path.dirname(torch.__file__)
+    cuda = os.path.dirname(os.path.dirname(_nvcc()))
+    inc = [os.path.join(root, "include"), os.path.join(root, "include", "torch", "csrc", "api", "include"),
+           sysconfig.get_paths()["include"], os.path.join(cuda, "include")]
+    return ["g++", "-O2", "-std=c++17", "-fPIC", "-shared", "-o", HOST_PATH, HOST_SOURCE, *["-I" + i for i in inc],
+            "-L" + os.path.join(root, "lib"), "-lc10", "-lc10_cuda", "-ltorch_cpu", "-ltorch_cuda", "-ltorch", "-ltorch_python"]
 
 
 def build_library(force: bool = False, verbose: bool = False) -> str:
-    """Compile if the shared object is missing or older than its sources; return its path."""
-    if not force and not is_stale():
-        return LIB_PATH
+    """Compile what is missing or older than its sources; return the library's path."""
+    host = None
     os.makedirs(LIB_DIR, exist_ok=True)
+    if force or _older(HOST_PATH, [HOST_SOURCE, HEADERS[-1]]):
+        env = {k: v for k, v in os.environ.items() if k not in ("CC", "CXX")}
+        host = subprocess.Popen(_host_command(), env=env)               # beside nvcc
+    try:
+        if force or is_stale():
+            _build_cuda(verbose)
+    finally:
+        if host is not None and host.wait() != 0:
+            raise RuntimeError("building hbq_host.so failed")
+    return LIB_PATH
+
+
+def _build_cuda(verbose: bool) -> None:
     cmd = [_nvcc(), *NVCC_FLAGS, "-o", LIB_PATH, *[os.path.join(CSRC, s) for s in SOURCES]]
     if verbose:
         cmd.insert(1, "-Xptxas")
@@ -52,7 +78,6 @@ def build_library(force: bool = False, verbose: bool = False) -> str:
     env.pop("CC", None)
     env.pop("CXX", None)
     subprocess.check_call(cmd, env=env)
-    return LIB_PATH
 
 
 if __name__ == "__main__":

@@ -16,6 +16,13 @@ def gemm(a: torch.Tensor, b: torch.Tensor, mode: int, group_k: int = 0, group_n:
          out: Optional[torch.Tensor] = None) -> torch.Tensor:
     """``hbq_gemm``: a [M, K] fp16, b [K, N] (or [N, K] when ``b_is_nk``) fp16 -> [M, N] fp16.
     ``out``: write into this contiguous fp16 [M, N] tensor instead of a new one."""
+    if out is None and not force_simt:
+        c = _lib.host().gemm(a, b, mode, group_k, group_n, bias, b_is_nk)
+        if c is not None:
+            if type(c) is int:
+                _lib.check(c, "hbq_gemm")
+            return c
+    # operands that need a conversion, a check or an output of the caller's
     if a.dtype != torch.float16 or b.dtype != torch.float16:
         raise RuntimeError("A must be fp16" if a.dtype != torch.float16 else "B must be fp16")
     if a.dim() != 2 or b.dim() != 2:

@@ -77,6 +77,12 @@ class W4Weight:
     def matmul(self, x: torch.Tensor, bias: Optional[torch.Tensor] = None, out: Optional[torch.Tensor] = None) -> torch.Tensor:
         """``x [M, K] fp16 -> x @ w.T (+ bias) [M, N] fp16``, M <= 128."""
         N, K = self.shape
+        if out is None and x.dim() == 2 and 0 < x.shape[0] <= MAX_ROWS:
+            c = _lib.host().gemm_w4(x, self.data, N, K, bytes(self.fmt), self.container_bits, bias, self._workspace(x.shape[0]))
+            if c is not None:
+                if type(c) is int:
+                    _lib.check(c, "hbq_gemm_w4")
+                return c
         if x.dtype != torch.float16 or x.dim() != 2 or x.shape[1] != K or x.device != self.data.device:
             raise RuntimeError("x must be an fp16 [M, K] tensor on the weight's device")
         M = x.shape[0]

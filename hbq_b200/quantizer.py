@@ -17,6 +17,7 @@ with ``x``'s shape and dtype, bit-identical to the reference's eager fp16 result
 from __future__ import annotations
 
 import ctypes
+import functools
 from dataclasses import dataclass
 from typing import Optional
 
@@ -89,7 +90,18 @@ class PackedTensor:
 
 
 def _stream_ptr(device) -> int:
-    return torch.cuda.current_stream(device).cuda_stream
+    return torch.cuda.current_stream(device).cuda_stream if device.index is None else _lib.host().current_stream(device.index)
+
+
+@functools.lru_cache(maxsize=256, typed=True)
+def _format_bytes(kind, ebit, mbit, sc_ebit, sc_mbit, block_size, allow_subnormal, use_round, use_ceil, l2_block_size,
+                  l2_sc_bit, l2_scheme, per_tensor_scale) -> bytes:
+    """An ``hbq_format`` as bytes, kept per field values: building the structure costs more than launching a kernel."""
+    return bytes(_lib.Format(kind, ebit, mbit, sc_ebit, sc_mbit, block_size, int(allow_subnormal), int(use_round), int(use_ceil),
+                             l2_block_size, l2_sc_bit, _lib.L2_SCHEMES.index(l2_scheme), int(per_tensor_scale), 0))
+
+
+_OUT_DTYPES = {None: -1, torch.float16: _lib.DTYPE_F16, torch.bfloat16: _lib.DTYPE_BF16}
 
 
 def _dtype_code(t: torch.Tensor) -> int:
@@ -177,8 +189,17 @@ class _CudaBlockQuantizer(_QBase):
         _lib.check(rc, f"hbq_quantize[{type(self).__name__}]")
         return deq
 
+    def _fmt_bytes(self) -> bytes:
+        return bytes(self._format())
+
     def q(self, x: torch.Tensor) -> torch.Tensor:
-        return self._launch(x, True, None)          # allocated with x's shape
+        odt = _OUT_DTYPES.get(self.out_dtype)
+        y = _lib.host().quantize(x, self._fmt_bytes(), odt) if odt is not None else None
+        if y is None:                               # anything but a plain contiguous fp16 / bf16 CUDA tensor
+            return self._launch(x, True, None)      # allocated with x's shape
+        if type(y) is int:
+            _lib.check(y, f"hbq_quantize[{type(self).__name__}]")
+        return y
 
     def quantize_packed(self, x: torch.Tensor, with_deq: bool = False):
         """Quantise ``x`` along its last axis into packed codes and scales.
@@ -232,6 +253,12 @@ class MXINTQuantizer(_CudaBlockQuantizer):
         return _lib.Format(_lib.KIND_MXINT, 0, self.nbit, self.sc_ebit, self.sc_mbit, self.block_size,
                            int(self.scale_allow_subnormal), 0, int(self.use_ceil), 0, 0, 0, 0, 0)
 
+    def _fmt_bytes(self):
+        if type(self) is not MXINTQuantizer:        # a subclass may have a format of its own
+            return bytes(self._format())
+        return _format_bytes(_lib.KIND_MXINT, 0, self.nbit, self.sc_ebit, self.sc_mbit, self.block_size,
+                             self.scale_allow_subnormal, 0, self.use_ceil, 0, 0, "PoT", 0)
+
 
 class MXFPQuantizer(_CudaBlockQuantizer):
     """MXFP / NVFP quantization (src/quantizer.py:430-539).
@@ -259,6 +286,12 @@ class MXFPQuantizer(_CudaBlockQuantizer):
         return _lib.Format(_lib.KIND_MXFP, self.ebit, self.mbit, self.sc_ebit, self.sc_mbit, self.block_size,
                            int(self.scale_allow_subnormal), int(self.use_round), int(self.use_ceil),
                            0, 0, 0, int(self.per_tensor_scale), 0)
+
+    def _fmt_bytes(self):
+        if type(self) is not MXFPQuantizer:
+            return bytes(self._format())
+        return _format_bytes(_lib.KIND_MXFP, self.ebit, self.mbit, self.sc_ebit, self.sc_mbit, self.block_size,
+                             self.scale_allow_subnormal, self.use_round, self.use_ceil, 0, 0, "PoT", self.per_tensor_scale)
 
 
 class HBQQuantizer(MXFPQuantizer):
@@ -289,6 +322,12 @@ class HBQQuantizer(MXFPQuantizer):
         return _lib.Format(_lib.KIND_HBQ, self.ebit, self.mbit, self.sc_ebit, self.sc_mbit, self.block_size,
                            int(self.scale_allow_subnormal), 0, int(self.use_ceil), self.l2_block_size,
                            self.l2_sc_bit, self.L2_SCHEME.index(self.l2_scheme), 0, 0)
+
+    def _fmt_bytes(self):
+        if type(self) is not HBQQuantizer:
+            return bytes(self._format())
+        return _format_bytes(_lib.KIND_HBQ, self.ebit, self.mbit, self.sc_ebit, self.sc_mbit, self.block_size,
+                             self.scale_allow_subnormal, 0, self.use_ceil, self.l2_block_size, self.l2_sc_bit, self.l2_scheme, 0)
 
     def l2_table(self, device=None) -> torch.Tensor:
         """Candidate micro-scales [n_scheme, 2**l2_sc_bit] (src/quantizer.py:745-770)."""

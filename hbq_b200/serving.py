@@ -138,13 +138,16 @@ class HBQLinearMethod:
         xq = self.act_quantizer.q(x)
         w4 = getattr(layer, "hbq_w4_weight", None)
         if w4 is not None and (layer.weight.numel() == 0 or xq.numel() // xq.shape[-1] <= self.packed_max_rows):
-            x2d = xq.reshape(-1, xq.shape[-1])
+            x2d = xq if xq.dim() == 2 else xq.reshape(-1, xq.shape[-1])
+            if 0 < x2d.shape[0] <= 128:
+                y = w4.matmul(x2d, bias)
+                return y if x.dim() == 2 else y.view(*x.shape[:-1], w4.shape[0])
             y = torch.empty((x2d.shape[0], w4.shape[0]), dtype=torch.float16, device=x2d.device)
             for r0 in range(0, x2d.shape[0], 128):
                 w4.matmul(x2d[r0:r0 + 128], bias, out=y[r0:r0 + 128])
             return y.view(*x.shape[:-1], w4.shape[0])
         w = layer.weight
         if xq.is_cuda and xq.dtype == torch.float16 and w.dtype == torch.float16:
-            y = ext.gemm_fp32_accum(xq.reshape(-1, xq.shape[-1]), w, b_is_nk=True, bias=bias)
-            return y.view(*x.shape[:-1], w.shape[0])
+            y = ext.gemm_fp32_accum(xq if xq.dim() == 2 else xq.reshape(-1, xq.shape[-1]), w, b_is_nk=True, bias=bias)
+            return y if x.dim() == 2 else y.view(*x.shape[:-1], w.shape[0])
         return torch.nn.functional.linear(xq, w, bias)
