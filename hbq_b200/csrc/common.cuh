@@ -80,6 +80,35 @@ inline int resident_ctas(Kernel kernel, int threads, size_t smem, int* ctas)
     return resident_ctas_impl(reinterpret_cast<const void*>(kernel), threads, smem, ctas);
 }
 
+// Programmatic dependent launch: a kernel launched with launch_dependent may start while the kernel before it in the
+// stream still runs -- once all of that kernel's CTAs have called dependents_may_start(), or have exited -- and does its
+// set-up (tables, barriers, tensor memory, prefetches into L2) until grid_dependency_wait(), which returns when that
+// kernel has completed and its writes are visible.  The rules that make the overlap safe: every thread waits before it
+// touches anything an earlier kernel may have written or may still read (L2 prefetches are exempt: L2 is where all of it
+// meets), and a kernel lets its dependents start only after its own wait, so that everything before it has completed.
+// HBQ-A activations [8, 4096] one after the other: 3.1 -> 2.3 us a call; quantizer and packed product of 8 rows x
+// [14336, 4096] 24.6 -> 18.5 us, of 33 x [4096, 14336] 31.9 -> 26.5 us.
+__device__ __forceinline__ void grid_dependency_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+__device__ __forceinline__ void dependents_may_start() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+// The pointer, made opaque behind the wait: loads through the read-only path may otherwise be moved above it.
+template <class T>
+__device__ __forceinline__ T* behind_wait(T* p)
+{
+    asm volatile("" : "+l"(p) :: "memory");
+    return p;
+}
+template <class... Params, class... Args>
+inline cudaError_t launch_dependent(void (*kernel)(Params...), dim3 grid, dim3 block, size_t smem, cudaStream_t stream, Args&&... args)
+{
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = grid; cfg.blockDim = block; cfg.dynamicSmemBytes = smem; cfg.stream = stream;
+    cudaLaunchAttribute at[1] = {};
+    at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at[0].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = at; cfg.numAttrs = 1;
+    return cudaLaunchKernelEx(&cfg, kernel, static_cast<Params>(args)...);
+}
+
 __device__ __forceinline__ uint32_t h2_bits(__half2 h) { return *reinterpret_cast<uint32_t*>(&h); }
 __device__ __forceinline__ __half2 bits_h2(uint32_t u) { return *reinterpret_cast<__half2*>(&u); }
 __device__ __forceinline__ uint16_t h_bits(__half h) { return __half_as_ushort(h); }

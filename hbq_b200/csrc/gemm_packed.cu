@@ -106,6 +106,8 @@ struct PkArgs {
     int split;                  // S >= 2: a tile's K range is split over the S CTAs of a cluster; 0: no clusters
 };
 
+__device__ __forceinline__ void l2_prefetch(const void* p) { asm volatile("prefetch.global.L2 [%0];" ::"l"(p)); }
+
 __device__ __forceinline__ uint32_t prmt(uint32_t a, uint32_t b, uint32_t sel)
 {
     uint32_t d;
@@ -307,9 +309,17 @@ gemm_packed_kernel(const __grid_constant__ CUtensorMap mapX, const __grid_consta
                      ::"r"(smem_u32(tmem_base_smem)), "r"(a.tmem_cols) : "memory");
         asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
     }
+    // the packed records of this CTA's run (one stretch of memory) on their way into L2 while the kernel before this one
+    // still runs
+    if (CB != 16 && warp == 6)
+        for (int i = lane; i < nst; i += 32)
+            asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;"
+                         ::"l"(a.wp + (int64_t)(g0 + i) * pk_rec_bytes(CB)), "r"(pk_rec_bytes(CB)) : "memory");
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
+    grid_dependency_wait();
+    dependents_may_start();
     const uint32_t tmem_base = *tmem_base_smem;
 
     if (warp == 4) {
@@ -793,8 +803,18 @@ __global__ void __launch_bounds__(512) gemv_packed_kernel(const GvArgs a)
     uint4* xs = reinterpret_cast<uint4*>(gv_smem);                               // [MT][K] fp16
     float* red = reinterpret_cast<float*>(gv_smem + (size_t)MT * a.K * 2);        // [ks][MT][32]
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    // while the kernel before this one (the tokens' quantizer) still runs: this CTA's weight on its way into L2 -- 32
+    // rows of every record, four runs of 512 bytes of codes and one of 256 of side words
+    for (int k = warp; k < a.nblk; k += a.ks) {
+        const uint8_t* rec = a.wp + ((int64_t)(blockIdx.x >> 2) * a.nblk + k) * pk_rec_bytes(4);
+        const int r0 = (blockIdx.x & 3) * 32;
+        if (lane < 16) l2_prefetch(rec + ((lane >> 2) * PK_ROWS + r0) * 16 + (lane & 3) * 128);
+        else if (lane < 18) l2_prefetch(rec + pk_code_bytes(4) + r0 * 8 + (lane & 1) * 128);
+    }
+    grid_dependency_wait();
+    dependents_may_start();
     {
-        const uint4* src = reinterpret_cast<const uint4*>(a.x);
+        const uint4* src = behind_wait(reinterpret_cast<const uint4*>(a.x));
         const int n16 = a.M * a.K / 8;
         for (int i = threadIdx.x; i < MT * a.K / 8; i += blockDim.x) xs[i] = i < n16 ? __ldg(src + i) : make_uint4(0u, 0u, 0u, 0u);
     }
@@ -901,6 +921,14 @@ __global__ void __launch_bounds__(512) gemm_packed_reg_kernel(const RgArgs a)
     const int slab = warp % a.slabs, ksp = warp / a.slabs;
     const int row0 = (blockIdx.x * a.slabs + slab) * 32, tile = row0 >> 7, rt = row0 & (PK_ROWS - 1);
     const uint8_t* rec0 = a.wp + (int64_t)tile * a.nblk * pk_rec_bytes(4);
+    for (int k = ksp; k < a.nblk; k += a.ks) {                                  // as in gemv_packed_kernel
+        const uint8_t* rec = rec0 + (int64_t)k * pk_rec_bytes(4);
+        if (lane < 16) l2_prefetch(rec + ((lane >> 2) * PK_ROWS + rt) * 16 + (lane & 3) * 128);
+        else if (lane < 18) l2_prefetch(rec + pk_code_bytes(4) + rt * 8 + (lane & 1) * 128);
+    }
+    grid_dependency_wait();
+    dependents_may_start();
+    const __half* const xin = behind_wait(a.x);
     float c[2][NT][4];
     #pragma unroll
     for (int G2 = 0; G2 < 2; ++G2)
@@ -940,7 +968,7 @@ __global__ void __launch_bounds__(512) gemm_packed_reg_kernel(const RgArgs a)
             #pragma unroll
             for (int nt = 0; nt < NT; ++nt) {
                 const int n = g + 8 * nt;
-                xv[q][nt] = n < a.M ? __ldg(reinterpret_cast<const uint4*>(a.x + (int64_t)n * a.K + kb * PK_KB + 32 * t + 8 * q))
+                xv[q][nt] = n < a.M ? __ldg(reinterpret_cast<const uint4*>(xin + (int64_t)n * a.K + kb * PK_KB + 32 * t + 8 * q))
                                     : make_uint4(0u, 0u, 0u, 0u);
             }
         #pragma unroll
@@ -1133,13 +1161,16 @@ static int launch_packed(const CUtensorMap& mx, const CUtensorMap& mw, const PkA
         cudaLaunchConfig_t cfg;
         memset(&cfg, 0, sizeof(cfg));
         cfg.gridDim = dim3((unsigned)grid); cfg.blockDim = dim3(PK_THREADS); cfg.dynamicSmemBytes = smem; cfg.stream = stream;
-        cudaLaunchAttribute at[1];
+        cudaLaunchAttribute at[2];
+        memset(at, 0, sizeof(at));
         at[0].id = cudaLaunchAttributeClusterDimension;
         at[0].val.clusterDim.x = (unsigned)a.split; at[0].val.clusterDim.y = 1; at[0].val.clusterDim.z = 1;
-        cfg.attrs = at; cfg.numAttrs = 1;
+        at[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+        at[1].val.programmaticStreamSerializationAllowed = 1;
+        cfg.attrs = at; cfg.numAttrs = 2;
         HBQ_CUDA_TRY(cudaLaunchKernelEx(&cfg, gemm_packed_kernel<MS, CB>, mx, mw, a));
     } else {
-        gemm_packed_kernel<MS, CB><<<grid, PK_THREADS, smem, stream>>>(mx, mw, a);
+        HBQ_CUDA_TRY(launch_dependent(gemm_packed_kernel<MS, CB>, grid, PK_THREADS, smem, stream, mx, mw, a));
     }
     HBQ_LAUNCH_CHECK("gemm_packed_kernel");
     return HBQ_OK;
@@ -1309,7 +1340,7 @@ static int w4_launch_gemv(const void* X, const void* Wp, void* C, int64_t M, int
     const size_t smem = (size_t)K * 2 + (size_t)ks * 32 * 4;
     auto go = [&](auto kern) -> int {
         { const int rc = ensure_dynamic_smem(kern, smem); if (rc) return rc; }
-        kern<<<units, ks * 32, smem, stream>>>(a);
+        HBQ_CUDA_TRY(launch_dependent(kern, units, ks * 32, smem, stream, a));
         HBQ_LAUNCH_CHECK("gemv_packed_kernel");
         return HBQ_OK;
     };
@@ -1334,8 +1365,7 @@ static int w4_launch_reg(const void* X, const void* Wp, void* C, int64_t M, int6
     a.slabs = slabs; a.ks = ks;
     const int grid = (int)(N / (32 * slabs));
     const size_t smem = (size_t)ks * slabs * 32 * 8 * 4;
-    if (ms == 0) gemm_packed_reg_kernel<0><<<grid, ks * slabs * 32, smem, stream>>>(a);
-    else gemm_packed_reg_kernel<2><<<grid, ks * slabs * 32, smem, stream>>>(a);
+    HBQ_CUDA_TRY(launch_dependent(ms == 0 ? gemm_packed_reg_kernel<0> : gemm_packed_reg_kernel<2>, grid, ks * slabs * 32, smem, stream, a));
     HBQ_LAUNCH_CHECK("gemm_packed_reg_kernel");
     return HBQ_OK;
 }

@@ -221,6 +221,8 @@ __device__ __forceinline__ void gemm_tc_body(const CUtensorMap& mapA, const Tile
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
+    grid_dependency_wait();
+    dependents_may_start();
     const uint32_t tmem_base = *tmem_base_smem;
 
     const int total_tiles = sched.total();
@@ -441,10 +443,12 @@ gemm_tc_grouped_kernel(const __grid_constant__ CUtensorMap mapA, const __grid_co
                        const __grid_constant__ TcArgs args)
 {
     __shared__ int s_first[TC_MAX_ENTRIES + 1], s_rows[2 * TC_MAX_ENTRIES];
+    grid_dependency_wait();
     if (threadIdx.x == 0) {
+        const int* const offsets = behind_wait(group.offsets);
         int n = 0;
         for (int e = 0; e < group.entries; ++e) {
-            const int r0 = __ldg(group.offsets + group.expert[e]), r1 = __ldg(group.offsets + group.expert[e] + 1);
+            const int r0 = offsets[group.expert[e]], r1 = offsets[group.expert[e] + 1];
             s_first[e] = n;
             s_rows[2 * e] = r0;
             s_rows[2 * e + 1] = r1;
@@ -553,10 +557,10 @@ static int launch_tc(const CUtensorMap& ma, const CUtensorMap& mb, const TcArgs&
 {
     if (args.bn == 128) {
         { const int rc = ensure_dynamic_smem(gemm_tc_kernel<MODE, GN, 128, 6>, smem_bytes(128, 6)); if (rc) return rc; }
-        gemm_tc_kernel<MODE, GN, 128, 6><<<grid, NTHREADS, smem_bytes(128, 6), stream>>>(ma, mb, args);
+        HBQ_CUDA_TRY(launch_dependent(gemm_tc_kernel<MODE, GN, 128, 6>, grid, NTHREADS, smem_bytes(128, 6), stream, ma, mb, args));
     } else {
         { const int rc = ensure_dynamic_smem(gemm_tc_kernel<MODE, GN, 256, 4>, smem_bytes(256, 4)); if (rc) return rc; }
-        gemm_tc_kernel<MODE, GN, 256, 4><<<grid, NTHREADS, smem_bytes(256, 4), stream>>>(ma, mb, args);
+        HBQ_CUDA_TRY(launch_dependent(gemm_tc_kernel<MODE, GN, 256, 4>, grid, NTHREADS, smem_bytes(256, 4), stream, ma, mb, args));
     }
     HBQ_LAUNCH_CHECK("gemm_tc_kernel");
     return HBQ_OK;
@@ -641,10 +645,10 @@ static int launch_grouped(const CUtensorMap& ma, const GroupArgs& g, const TcArg
 {
     if (args.bn == 128) {
         { const int rc = ensure_dynamic_smem(gemm_tc_grouped_kernel<MODE, GN, 128, 6>, smem_bytes(128, 6)); if (rc) return rc; }
-        gemm_tc_grouped_kernel<MODE, GN, 128, 6><<<grid, NTHREADS, smem_bytes(128, 6), stream>>>(ma, g, args);
+        HBQ_CUDA_TRY(launch_dependent(gemm_tc_grouped_kernel<MODE, GN, 128, 6>, grid, NTHREADS, smem_bytes(128, 6), stream, ma, g, args));
     } else {
         { const int rc = ensure_dynamic_smem(gemm_tc_grouped_kernel<MODE, GN, 256, 4>, smem_bytes(256, 4)); if (rc) return rc; }
-        gemm_tc_grouped_kernel<MODE, GN, 256, 4><<<grid, NTHREADS, smem_bytes(256, 4), stream>>>(ma, g, args);
+        HBQ_CUDA_TRY(launch_dependent(gemm_tc_grouped_kernel<MODE, GN, 256, 4>, grid, NTHREADS, smem_bytes(256, 4), stream, ma, g, args));
     }
     HBQ_LAUNCH_CHECK("gemm_tc_grouped_kernel");
     return HBQ_OK;

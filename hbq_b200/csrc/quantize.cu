@@ -308,9 +308,9 @@ __device__ __forceinline__ void mx_fast_chunk(const QArgs& a, const Chunk& x, __
 // LEAN: the tensor is contiguous, 16-byte aligned, K a multiple of the block, and only the
 //        fake-quantised output is wanted: chunk ci is elements [8 ci, 8 ci + 8) of both tensors, so
 //        the row / column bookkeeping, RoPE / permutation and side outputs drop out.
-__device__ __forceinline__ Chunk lean_load(const QArgs& a, int64_t ci)
+__device__ __forceinline__ Chunk lean_load(const QArgs& a, const uint4* x, int64_t ci)
 {
-    const uint4 v = __ldg(reinterpret_cast<const uint4*>(a.x) + ci);
+    const uint4 v = __ldg(x + ci);
     const uint32_t w[4] = {v.x, v.y, v.z, v.w};
     Chunk c;
     if (!a.in_bf16) {
@@ -332,13 +332,19 @@ __global__ void __launch_bounds__(256, LEAN ? 8 : 1) mx_fast_kernel(const QArgs 
 {
     // Grid-stride loop with the next chunk's load issued before the current one is processed, so
     // every thread keeps a 16-byte load in flight while it computes.
+    const uint4* xin = nullptr;
+    if (LEAN) {                              // (launched as a dependent in this form only)
+        grid_dependency_wait();
+        dependents_may_start();
+        xin = behind_wait(reinterpret_cast<const uint4*>(a.x));
+    }
     const int lane = threadIdx.x & 31;
     const int64_t stride = (int64_t)gridDim.x * blockDim.x;
     int64_t ci = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     int64_t row = 0, c = 0;
     if (!LEAN) split_chunk(a, ci < a.total_chunks ? ci : 0, row, c);
     Chunk x;
-    if (ci < a.total_chunks) x = LEAN ? lean_load(a, ci) : load_chunk(a, row, c * 8);
+    if (ci < a.total_chunks) x = LEAN ? lean_load(a, xin, ci) : load_chunk(a, row, c * 8);
     else { for (int p = 0; p < 4; ++p) x.h[p] = bits_h2(0u); }
     for (; ci - lane < a.total_chunks; ci += stride) {
     const bool valid = ci < a.total_chunks;
@@ -350,7 +356,7 @@ __global__ void __launch_bounds__(256, LEAN ? 8 : 1) mx_fast_kernel(const QArgs 
         if (c >= a.cpr) { c -= a.cpr; ++row; }
     }
     Chunk xn;
-    if (ci + stride < a.total_chunks) xn = LEAN ? lean_load(a, ci + stride) : load_chunk(a, row, c * 8);
+    if (ci + stride < a.total_chunks) xn = LEAN ? lean_load(a, xin, ci + stride) : load_chunk(a, row, c * 8);
     else { for (int p = 0; p < 4; ++p) xn.h[p] = bits_h2(0u); }
 
     if (!LEAN && a.rope_cos) rope_chunk(a, x, valid ? row_cur : 0, k0);
@@ -739,7 +745,8 @@ static int launch_mx_fast_as(QArgs& a, dim3 grid, dim3 block, cudaStream_t strea
     const int64_t stride = (int64_t)grid.x * block.x;
     a.step_rows = stride / a.cpr;
     a.step_chunks = stride % a.cpr;
-    mx_fast_kernel<KIND, MB, CODES, LEAN><<<grid, block, 0, stream>>>(a);
+    if (LEAN) HBQ_CUDA_TRY(launch_dependent(mx_fast_kernel<KIND, MB, CODES, LEAN>, grid, block, 0, stream, a));
+    else mx_fast_kernel<KIND, MB, CODES, LEAN><<<grid, block, 0, stream>>>(a);
     return HBQ_OK;
 }
 

@@ -369,16 +369,16 @@ __device__ __forceinline__ void store_block_side(const TabArgs& a, int64_t bi, i
 // so chunk k's rotation partner (d +- D/2) is chunk k +- C/2 of the same thread.  Every product, the sum and the
 // difference are rounded to fp16 like the reference's tensor ops (the _rn forms keep ptxas from contracting them).
 template <int C>
-__device__ __forceinline__ void kv_rows(const TabArgs& a, uint32_t (*xb)[4], uint32_t bt, uint32_t b, uint32_t t, uint32_t h,
+__device__ __forceinline__ void kv_rows(const TabArgs& a, const uint4* rope_cos, const uint4* rope_sin, const uint4* center, uint32_t (*xb)[4], uint32_t bt, uint32_t b, uint32_t t, uint32_t h,
                                         int Gt, int g)
 {
     const int cpr = C * Gt;
-    if (a.rope_cos) {
+    if (rope_cos) {
         const int64_t r0 = (int64_t)(a.rope_rows == a.kv_T ? t : bt % a.rope_rows) * cpr + g;
         #pragma unroll
         for (int k = 0; k < C / 2; ++k) {
-            const uint4 c0 = __ldg(a.rope_cos + r0 + k * Gt), s0 = __ldg(a.rope_sin + r0 + k * Gt);
-            const uint4 c1 = __ldg(a.rope_cos + r0 + (k + C / 2) * Gt), s1 = __ldg(a.rope_sin + r0 + (k + C / 2) * Gt);
+            const uint4 c0 = __ldg(rope_cos + r0 + k * Gt), s0 = __ldg(rope_sin + r0 + k * Gt);
+            const uint4 c1 = __ldg(rope_cos + r0 + (k + C / 2) * Gt), s1 = __ldg(rope_sin + r0 + (k + C / 2) * Gt);
             const uint32_t cl[4] = {c0.x, c0.y, c0.z, c0.w}, sl[4] = {s0.x, s0.y, s0.z, s0.w};
             const uint32_t ch[4] = {c1.x, c1.y, c1.z, c1.w}, sh[4] = {s1.x, s1.y, s1.z, s1.w};
             #pragma unroll
@@ -389,11 +389,11 @@ __device__ __forceinline__ void kv_rows(const TabArgs& a, uint32_t (*xb)[4], uin
             }
         }
     }
-    if (a.center) {
+    if (center) {
         const int64_t r0 = ((int64_t)b * a.kv_H + h) * cpr + g;
         #pragma unroll
         for (int k = 0; k < C; ++k) {
-            const uint4 cv = __ldg(a.center + r0 + k * Gt);
+            const uint4 cv = __ldg(center + r0 + k * Gt);
             const uint32_t c[4] = {cv.x, cv.y, cv.z, cv.w};
             #pragma unroll
             for (int p = 0; p < 4; ++p) xb[k][p] = h2_bits(__hsub2_rn(bits_h2(xb[k][p]), bits_h2(c[p])));
@@ -414,6 +414,13 @@ __global__ void __launch_bounds__(TAB_THREADS, 2) hbq_tab_kernel(const TabArgs a
     __shared__ float s_tabf[4];
     const int tid = threadIdx.x, lane = tid & 31;
     const uint32_t dst = stage_table(a, s_tab, s_l1c, &s_bar, s_nt2, s_tabf, TAB_THREADS);
+    grid_dependency_wait();
+    dependents_may_start();
+    const uint4* const xin = behind_wait(a.x);
+    const uint4* const gin = GLU ? behind_wait(a.gate) : nullptr;
+    const uint4* const rope_cos = KV ? behind_wait(a.rope_cos) : nullptr;
+    const uint4* const rope_sin = KV ? behind_wait(a.rope_sin) : nullptr;
+    const uint4* const center = KV ? behind_wait(a.center) : nullptr;
 
     const int log2Gt = GT > 0 ? (GT == 1 ? 0 : GT == 2 ? 1 : GT == 4 ? 2 : GT == 8 ? 3 : GT == 16 ? 4 : 5) : a.log2Gt;
     const int Gt = 1 << log2Gt;
@@ -429,10 +436,10 @@ __global__ void __launch_bounds__(TAB_THREADS, 2) hbq_tab_kernel(const TabArgs a
         #pragma unroll
         for (int k = 0; k < C; ++k) {
             rx[k] = make_uint4(0u, 0u, 0u, 0u);
-            if (ok) rx[k] = __ldg(a.x + cc + k * Gt);
+            if (ok) rx[k] = __ldg(xin + cc + k * Gt);
             if (GLU) {
                 rg[k] = make_uint4(0u, 0u, 0u, 0u);
-                if (ok) rg[k] = __ldg(a.gate + cc + k * Gt);
+                if (ok) rg[k] = __ldg(gin + cc + k * Gt);
             }
         }
     };
@@ -472,7 +479,7 @@ __global__ void __launch_bounds__(TAB_THREADS, 2) hbq_tab_kernel(const TabArgs a
         if (KV) {
             const uint32_t row = valid ? (uint32_t)bi : 0u;
             const uint32_t bt = row / a.kv_H, h = row - bt * a.kv_H, b = bt / a.kv_T, t = bt - b * a.kv_T;
-            kv_rows<C>(a, xb, bt, b, t, h, Gt, g);
+            kv_rows<C>(a, rope_cos, rope_sin, center, xb, bt, b, t, h, Gt, g);
             o0 = (((int64_t)b * a.kv_H + h) * a.kv_T + t) * (C * Gt) + g;
         }
 
@@ -514,10 +521,10 @@ __global__ void __launch_bounds__(TAB_THREADS, 2) hbq_tab_kernel(const TabArgs a
             #pragma unroll
             for (int k = 0; k < C; ++k) {                  // unrolled: xb must stay in registers
                 const float tc = s_tabf[(bests >> (2 * k)) & 3u];
-                uint4 raw = __ldg(a.x + c0 + k * Gt);
+                uint4 raw = __ldg(xin + c0 + k * Gt);
                 uint32_t xr[4] = {raw.x, raw.y, raw.z, raw.w};
                 if (GLU) {
-                    const uint4 graw = __ldg(a.gate + c0 + k * Gt);
+                    const uint4 graw = __ldg(gin + c0 + k * Gt);
                     const uint32_t gb[4] = {graw.x, graw.y, graw.z, graw.w};
                     for (int p = 0; p < 4; ++p) {
                         const float2 gg = __half22float2(bits_h2(gb[p])), uu = __half22float2(bits_h2(xr[p]));
@@ -661,6 +668,9 @@ __global__ void __launch_bounds__(MIX_THREADS, 2) hbq_tab_mix_kernel(const TabAr
     __shared__ float s_tabf[8];
     const int tid = threadIdx.x, lane = tid & 31;
     const uint32_t dst = stage_table<true>(a, s_tab, s_l1c, &s_bar, s_nt2, s_tabf, MIX_THREADS);
+    grid_dependency_wait();
+    dependents_may_start();
+    const uint4* const xin = behind_wait(a.x);
     const int log2Gt = GT == 4 ? 2 : a.log2Gt;
     const int Gt = 1 << log2Gt;
     const int64_t stride = (int64_t)gridDim.x * MIX_THREADS;
@@ -675,7 +685,7 @@ __global__ void __launch_bounds__(MIX_THREADS, 2) hbq_tab_mix_kernel(const TabAr
         uint32_t xb[C][4];
         #pragma unroll
         for (int k = 0; k < C; ++k) {
-            const uint4 r = valid ? __ldg(a.x + c0 + k * Gt) : make_uint4(0u, 0u, 0u, 0u);
+            const uint4 r = valid ? __ldg(xin + c0 + k * Gt) : make_uint4(0u, 0u, 0u, 0u);
             xb[k][0] = r.x; xb[k][1] = r.y; xb[k][2] = r.z; xb[k][3] = r.w;
         }
         if (a.in_bf16) {
@@ -828,6 +838,9 @@ __global__ void __launch_bounds__(TABV_THREADS, 4) hbq_tab_v_kernel(const TabArg
     __shared__ float s_tabf[4];
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const uint32_t dst = stage_table(a, s_tab, s_l1c, &s_bar, s_nt2, s_tabf, TABV_THREADS);
+    grid_dependency_wait();
+    dependents_may_start();
+    const uint16_t* const vin = behind_wait(v.in);
     const int seg = tid & 7;                                     // load / store phases: 8 channels
     #pragma unroll 1
     for (int64_t tl = blockIdx.x; tl < v.tiles; tl += gridDim.x) {
@@ -838,7 +851,7 @@ __global__ void __launch_bounds__(TABV_THREADS, 4) hbq_tab_v_kernel(const TabArg
         const int64_t b = bh / v.H, h = bh - b * v.H;
         const int64_t t0 = (int64_t)tb * TABV_T;
         const int d0 = ds * TABV_D + seg * 8;
-        const uint16_t* src = v.in + ((b * v.T * v.H + h) * v.D + d0);
+        const uint16_t* src = vin + ((b * v.T * v.H + h) * v.D + d0);
 
         uint4 ld[4];
         #pragma unroll
@@ -1014,6 +1027,12 @@ __global__ void __launch_bounds__(ROW_THREADS, 2) hbq_row_kernel(const RowArgs a
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     uint32_t dst = 0u;
     if (QUANT) dst = stage_table(a.t, s_tab, s_l1c, &s_bar, s_nt2, s_tabf, ROW_THREADS);
+    grid_dependency_wait();
+    dependents_may_start();
+    const uint4* const ain = behind_wait(a.in);
+    const uint4* const ares = PRO == ROW_RMSNORM ? behind_wait(a.res) : nullptr;
+    const uint4* const aw = PRO == ROW_RMSNORM ? behind_wait(a.w) : nullptr;
+    const uint4* const amask = PRO == ROW_SOFTMAX ? behind_wait(a.mask) : nullptr;
     // RMSNorm: one row per warp, 8 blocks (1024 elements) per iteration.  Softmax: one row per half-warp, 4 blocks
     // per iteration -- a causal row ends anywhere, and the masked blocks of its last iteration are lanes without
     // work (1.5 blocks on average instead of 3.5).
@@ -1030,7 +1049,7 @@ __global__ void __launch_bounds__(ROW_THREADS, 2) hbq_row_kernel(const RowArgs a
         int64_t row = rb + sub;
         const bool live = row < a.rows;                      // odd row count: the idle half repeats the last row, stores nothing
         if (!live) row = a.rows - 1;
-        const uint4* rin = a.in + row * cpr;
+        const uint4* rin = ain + row * cpr;
         uint4* rout = a.out + row * cpr;
         float stat0 = 0.f, stat1 = 0.f;                      // RMSNORM: rstd; SOFTMAX: max, sum
         int iters = iters_all;
@@ -1041,7 +1060,7 @@ __global__ void __launch_bounds__(ROW_THREADS, 2) hbq_row_kernel(const RowArgs a
         if (PRO == ROW_RMSNORM) {
             float ss = 0.f;
             uint4* rx = a.x_out ? a.x_out + row * cpr : nullptr;
-            const uint4* rres = a.res ? a.res + row * cpr : nullptr;
+            const uint4* rres = ares ? ares + row * cpr : nullptr;
             if (rres) rsrc = rx;
             for (int it = 0; it < iters; ++it) {
                 const int blk = it * BPI + bl;
@@ -1072,7 +1091,7 @@ __global__ void __launch_bounds__(ROW_THREADS, 2) hbq_row_kernel(const RowArgs a
             const int64_t qpos = row % a.L;
             if (a.causal) limit = qpos + a.key_offset;
             if (limit > (int64_t)a.K - 1) limit = (int64_t)a.K - 1;
-            if (a.mask) rmask = a.mask + ((a.mask_batches > 1 ? row / a.HL : 0) * a.L + qpos) * cpr;
+            if (amask) rmask = amask + ((a.mask_batches > 1 ? row / a.HL : 0) * a.L + qpos) * cpr;
             // whole iterations beyond the causal limit hold only masked keys: probabilities 0
             iters = min(iters_all, (int)(limit / (128 * BPI)) + 1);
             float mx = -INFINITY;
@@ -1160,7 +1179,7 @@ __global__ void __launch_bounds__(ROW_THREADS, 2) hbq_row_kernel(const RowArgs a
                 if (blk >= a.nblk || ci >= cpr) continue;
                 if (PRO == ROW_RMSNORM) {
                     // weight * fp16(x_f32 * rstd): the rounding points of transformers' LlamaRMSNorm on an fp16 tensor
-                    const uint4 v = a.res ? rsrc[ci] : __ldg(rsrc + ci), wv = __ldg(a.w + ci);
+                    const uint4 v = ares ? rsrc[ci] : __ldg(rsrc + ci), wv = __ldg(aw + ci);
                     const uint32_t q[4] = {v.x, v.y, v.z, v.w}, ww[4] = {wv.x, wv.y, wv.z, wv.w};
                     #pragma unroll
                     for (int p = 0; p < 4; ++p) {
@@ -1248,7 +1267,7 @@ static int launch_tab(const TabArgs& a, size_t smem, cudaStream_t stream)
     { const int rc = ensure_dynamic_smem(hbq_tab_kernel<MB, C, GT, ML, SIDE, GLU, KV>, smem); if (rc) return rc; }
     { const int rc = resident_ctas(hbq_tab_kernel<MB, C, GT, ML, SIDE, GLU, KV>, TAB_THREADS, smem, &per_sm); if (rc) return rc; }
     const int grid = tab_grid(a.total_units, (int64_t)sms * per_sm);
-    hbq_tab_kernel<MB, C, GT, ML, SIDE, GLU, KV><<<grid, TAB_THREADS, smem, stream>>>(a);
+    HBQ_CUDA_TRY(launch_dependent(hbq_tab_kernel<MB, C, GT, ML, SIDE, GLU, KV>, grid, TAB_THREADS, smem, stream, a));
     HBQ_LAUNCH_CHECK("hbq_tab_kernel");
     return HBQ_OK;
 }
@@ -1268,7 +1287,7 @@ static int launch_mix(const TabArgs& a, size_t smem, cudaStream_t stream)
     { const int rc = device_sms(&sms); if (rc) return rc; }
     { const int rc = ensure_dynamic_smem(hbq_tab_mix_kernel<MB, GT, ML, SIDE>, smem); if (rc) return rc; }
     { const int rc = resident_ctas(hbq_tab_mix_kernel<MB, GT, ML, SIDE>, MIX_THREADS, smem, &per_sm); if (rc) return rc; }
-    hbq_tab_mix_kernel<MB, GT, ML, SIDE><<<tab_grid(a.total_units, (int64_t)sms * per_sm), MIX_THREADS, smem, stream>>>(a);
+    HBQ_CUDA_TRY(launch_dependent(hbq_tab_mix_kernel<MB, GT, ML, SIDE>, tab_grid(a.total_units, (int64_t)sms * per_sm), MIX_THREADS, smem, stream, a));
     HBQ_LAUNCH_CHECK("hbq_tab_mix_kernel");
     return HBQ_OK;
 }
@@ -1334,9 +1353,9 @@ static int launch_row(const RowArgs& a, bool quant, cudaStream_t stream)
     const int grid = (int)(need < 2ll * sms ? need : 2ll * sms);
     if (quant) {
         { const int rc = ensure_dynamic_smem(hbq_row_kernel<MB, ML, PRO, true>, smem); if (rc) return rc; }
-        hbq_row_kernel<MB, ML, PRO, true><<<grid, ROW_THREADS, smem, stream>>>(a);
+        HBQ_CUDA_TRY(launch_dependent(hbq_row_kernel<MB, ML, PRO, true>, grid, ROW_THREADS, smem, stream, a));
     } else {
-        hbq_row_kernel<MB, ML, PRO, false><<<grid, ROW_THREADS, 0, stream>>>(a);
+        HBQ_CUDA_TRY(launch_dependent(hbq_row_kernel<MB, ML, PRO, false>, grid, ROW_THREADS, 0, stream, a));
     }
     HBQ_LAUNCH_CHECK("hbq_row_kernel");
     return HBQ_OK;
@@ -1494,7 +1513,7 @@ static int launch_tab_v(const TabArgs& a, const VArgs& v, cudaStream_t stream)
     { const int rc = ensure_dynamic_smem(hbq_tab_v_kernel<MB, ML>, smem); if (rc) return rc; }
     { const int rc = resident_ctas(hbq_tab_v_kernel<MB, ML>, TABV_THREADS, smem, &per_sm); if (rc) return rc; }
     const int64_t cap = (int64_t)sms * per_sm;
-    hbq_tab_v_kernel<MB, ML><<<(int)(v.tiles < cap ? v.tiles : cap), TABV_THREADS, smem, stream>>>(a, v);
+    HBQ_CUDA_TRY(launch_dependent(hbq_tab_v_kernel<MB, ML>, (unsigned)(v.tiles < cap ? v.tiles : cap), TABV_THREADS, smem, stream, a, v));
     HBQ_LAUNCH_CHECK("hbq_tab_v_kernel");
     return HBQ_OK;
 }
