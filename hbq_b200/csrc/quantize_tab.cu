@@ -1045,7 +1045,9 @@ __global__ void __launch_bounds__(ROW_THREADS, 2) hbq_row_kernel(const RowArgs a
     const int iters_all = (a.nblk + BPI - 1) / BPI;
 
     #pragma unroll 1
-    for (int64_t rb = ((int64_t)blockIdx.x * ROW_WARPS + warp) * RPW; rb < a.rows; rb += (int64_t)gridDim.x * ROW_WARPS * RPW) {
+    // warps take turns over the CTAs: the rows of one CTA then lie far apart, so that causal rows of every length and the
+    // rows of a last partial round are spread over the SMs
+    for (int64_t rb = ((int64_t)warp * gridDim.x + blockIdx.x) * RPW; rb < a.rows; rb += (int64_t)gridDim.x * ROW_WARPS * RPW) {
         int64_t row = rb + sub;
         const bool live = row < a.rows;                      // odd row count: the idle half repeats the last row, stores nothing
         if (!live) row = a.rows - 1;
@@ -1348,8 +1350,8 @@ static int launch_row(const RowArgs& a, bool quant, cudaStream_t stream)
     int sms = 0;
     { const int rc = device_sms(&sms); if (rc) return rc; }
     const size_t smem = quant ? (size_t)a.t.entries * 4 : 0;
-    const int64_t rows_per_cta = ROW_WARPS * (PRO == ROW_SOFTMAX ? 2 : 1);
-    const int64_t need = (a.rows + rows_per_cta - 1) / rows_per_cta;
+    constexpr int RPW = PRO == ROW_SOFTMAX ? 2 : 1;
+    const int64_t need = (a.rows + RPW * TAB_MIN_WARPS - 1) / (RPW * TAB_MIN_WARPS);
     const int grid = (int)(need < 2ll * sms ? need : 2ll * sms);
     if (quant) {
         { const int rc = ensure_dynamic_smem(hbq_row_kernel<MB, ML, PRO, true>, smem); if (rc) return rc; }
