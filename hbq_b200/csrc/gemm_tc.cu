@@ -552,18 +552,36 @@ bool gemm_tc_eligible(int64_t M, int64_t N, int64_t K, int mode, int group_k, in
     return true;
 }
 
+// Tile width: all CTAs of a round work on tiles of one width, so the time is (rounds) x (width).  256 columns as a rule: a
+// narrower tile reads A again for less work and a column of it costs some 15 % more (forced to 192: 4096 x 4096 x 4096
+// 105 -> 119 us; to 224: 4096 x 14336 x 4096 343 -> 360 us, though both save 5 % of rounds x width).  192 where they take
+// no more rounds (1000 x 6144 x 4096, 192 tiles of 256 or 256 of 192 in two rounds of 148: fp32 53.8 -> 48.0 us, grouped
+// fp16 sums 59.6 -> 50.5), for the accumulation models whose drain of an accumulator is shorter than its MMAs; 128 where
+// 256-column tiles would leave more than half of the SMs without work, or for N of at most 128.
+static int tile_width(int64_t tiles_m, int64_t N, int sms, int mode)
+{
+    const int64_t t256 = tiles_m * ((N + 255) / 256), t192 = tiles_m * ((N + 191) / 192);
+    if (N <= 128 || t256 * 2 <= sms) return 128;
+    const bool light = mode == HBQ_ACC_FP32 || mode == HBQ_ACC_GROUPED;
+    return light && (t192 + sms - 1) / sms == (t256 + sms - 1) / sms ? 192 : 256;
+}
+
+template <int MODE, int GN, int BN, int NSTAGE>
+static int launch_tc_as(const CUtensorMap& ma, const CUtensorMap& mb, const TcArgs& args, int grid, cudaStream_t stream)
+{
+    { const int rc = ensure_dynamic_smem(gemm_tc_kernel<MODE, GN, BN, NSTAGE>, smem_bytes(BN, NSTAGE)); if (rc) return rc; }
+    HBQ_CUDA_TRY(launch_dependent(gemm_tc_kernel<MODE, GN, BN, NSTAGE>, grid, NTHREADS, smem_bytes(BN, NSTAGE), stream, ma, mb, args));
+    HBQ_LAUNCH_CHECK("gemm_tc_kernel");
+    return HBQ_OK;
+}
+
 template <int MODE, int GN>
 static int launch_tc(const CUtensorMap& ma, const CUtensorMap& mb, const TcArgs& args, int grid, cudaStream_t stream)
 {
-    if (args.bn == 128) {
-        { const int rc = ensure_dynamic_smem(gemm_tc_kernel<MODE, GN, 128, 6>, smem_bytes(128, 6)); if (rc) return rc; }
-        HBQ_CUDA_TRY(launch_dependent(gemm_tc_kernel<MODE, GN, 128, 6>, grid, NTHREADS, smem_bytes(128, 6), stream, ma, mb, args));
-    } else {
-        { const int rc = ensure_dynamic_smem(gemm_tc_kernel<MODE, GN, 256, 4>, smem_bytes(256, 4)); if (rc) return rc; }
-        HBQ_CUDA_TRY(launch_dependent(gemm_tc_kernel<MODE, GN, 256, 4>, grid, NTHREADS, smem_bytes(256, 4), stream, ma, mb, args));
+    if constexpr (MODE == HBQ_ACC_FP32 || MODE == HBQ_ACC_GROUPED) {
+        if (args.bn == 192) return launch_tc_as<MODE, GN, 192, 4>(ma, mb, args, grid, stream);
     }
-    HBQ_LAUNCH_CHECK("gemm_tc_kernel");
-    return HBQ_OK;
+    return args.bn == 128 ? launch_tc_as<MODE, GN, 128, 6>(ma, mb, args, grid, stream) : launch_tc_as<MODE, GN, 256, 4>(ma, mb, args, grid, stream);
 }
 
 int transpose_launch(const void* in, void* out, int64_t R, int64_t Ccols, cudaStream_t stream)
@@ -597,9 +615,7 @@ int gemm_tc_launch_ex(const void* A, const void* W, void* C, int64_t M, int64_t 
     int sms = 0;
     { const int rc2 = device_sms(&sms); if (rc2) return rc2; }
     args.tiles_m = (int)((M + BM - 1) / BM);
-    // 128-column tiles when 256-column ones would leave more than half of the SMs without work
-    // ... or when the whole problem is at most 128 columns wide (a 256-column tile would be half empty)
-    args.bn = (N <= 128 || (int64_t)args.tiles_m * ((N + 255) / 256) * 2 <= sms) ? 128 : 256;
+    args.bn = tile_width(args.tiles_m, N, sms, mode);
     args.tiles_n = (int)((N + args.bn - 1) / args.bn);
     rc = make_map(&mb, W, N, K, args.bn);
     if (rc) return rc;
@@ -640,18 +656,22 @@ int gemm_tc_launch(const void* A, const void* W, void* C, int64_t M, int64_t N, 
     return gemm_tc_launch_ex(A, W, C, M, N, K, mode, group_k, group_n, bias, stream, 0, 0);
 }
 
+template <int MODE, int GN, int BN, int NSTAGE>
+static int launch_grouped_as(const CUtensorMap& ma, const GroupArgs& g, const TcArgs& args, int grid, cudaStream_t stream)
+{
+    { const int rc = ensure_dynamic_smem(gemm_tc_grouped_kernel<MODE, GN, BN, NSTAGE>, smem_bytes(BN, NSTAGE)); if (rc) return rc; }
+    HBQ_CUDA_TRY(launch_dependent(gemm_tc_grouped_kernel<MODE, GN, BN, NSTAGE>, grid, NTHREADS, smem_bytes(BN, NSTAGE), stream, ma, g, args));
+    HBQ_LAUNCH_CHECK("gemm_tc_grouped_kernel");
+    return HBQ_OK;
+}
+
 template <int MODE, int GN>
 static int launch_grouped(const CUtensorMap& ma, const GroupArgs& g, const TcArgs& args, int grid, cudaStream_t stream)
 {
-    if (args.bn == 128) {
-        { const int rc = ensure_dynamic_smem(gemm_tc_grouped_kernel<MODE, GN, 128, 6>, smem_bytes(128, 6)); if (rc) return rc; }
-        HBQ_CUDA_TRY(launch_dependent(gemm_tc_grouped_kernel<MODE, GN, 128, 6>, grid, NTHREADS, smem_bytes(128, 6), stream, ma, g, args));
-    } else {
-        { const int rc = ensure_dynamic_smem(gemm_tc_grouped_kernel<MODE, GN, 256, 4>, smem_bytes(256, 4)); if (rc) return rc; }
-        HBQ_CUDA_TRY(launch_dependent(gemm_tc_grouped_kernel<MODE, GN, 256, 4>, grid, NTHREADS, smem_bytes(256, 4), stream, ma, g, args));
+    if constexpr (MODE == HBQ_ACC_FP32 || MODE == HBQ_ACC_GROUPED) {
+        if (args.bn == 192) return launch_grouped_as<MODE, GN, 192, 4>(ma, g, args, grid, stream);
     }
-    HBQ_LAUNCH_CHECK("gemm_tc_grouped_kernel");
-    return HBQ_OK;
+    return args.bn == 128 ? launch_grouped_as<MODE, GN, 128, 6>(ma, g, args, grid, stream) : launch_grouped_as<MODE, GN, 256, 4>(ma, g, args, grid, stream);
 }
 
 // A [rows, K]; entry i: C[i][r, :] = A[r, :] * W[i][N, K]^T for the rows offsets[expert[i]] .. offsets[expert[i] + 1] - 1
@@ -671,10 +691,13 @@ int gemm_tc_grouped_launch(const void* A, int64_t rows, const int* offsets, int 
     TcArgs args;
     memset(&args, 0, sizeof(args));
     args.M = (int)rows; args.N = (int)N; args.K = (int)K;
-    // 128-column tiles, as for one product, where even one row tile per entry and the rows' own tiles of 256 columns
-    // would leave more than half of the SMs without work
-    const int64_t tiles256 = ((rows < entries ? rows : entries) + rows / BM) * ((N + 255) / 256);
-    args.bn = (N <= 128 || tiles256 * 2 <= sms) ? 128 : 256;
+    // the row tiles are known on the device only: every entry's rows end inside a tile, half a tile on average
+    const int n0 = entries < TC_MAX_ENTRIES ? entries : TC_MAX_ENTRIES;
+    int experts = 1;
+    for (int i = 0; i < entries; ++i) experts = experts > expert[i] + 1 ? experts : expert[i] + 1;
+    const int64_t rows_tiles = rows < experts ? rows : rows / BM + (experts + 1) / 2;
+    const int64_t tiles_m = rows_tiles * n0 / experts > 0 ? rows_tiles * n0 / experts : 1;
+    args.bn = tile_width(tiles_m, N, sms, mode);
     args.tiles_n = (int)((N + args.bn - 1) / args.bn);
     args.k_stages = (int)((K + BK - 1) / BK);
     args.chunk_k16 = (mode == HBQ_ACC_FP32) ? args.k_stages * (BK / 16) : group_k / 16;
