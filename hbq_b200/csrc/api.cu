@@ -120,6 +120,30 @@ int hbq_kv_write_k(const void* k, int dtype, int64_t B, int64_t T, int64_t H, in
     return quantize_launch(k, dtype, B * T * H, D, fmt, out, out_dtype, nullptr, nullptr, (cudaStream_t)stream, &kv);
 }
 
+int hbq_quantize_q_runs(const void* q, int64_t B, int64_t T, int64_t H, int64_t D, int64_t run, int64_t group, const void* cos,
+                        const void* sin, int64_t rope_rows, const hbq_format* fmt, void* out, void* stream)
+{
+    if (!fmt || B < 0 || T < 0 || H <= 0 || D <= 0 || run <= 0 || group <= 0 || T % run || H % group || !cos || !sin) return HBQ_ERR_ARG;
+    if (B * T == 0) return HBQ_OK;
+    if (!out) return HBQ_ERR_ARG;
+    if (fmt->kind == HBQ_KIND_MXFP && fmt->per_tensor_scale) return HBQ_ERR_UNSUPPORTED;
+    KvWriteOpts kv = {cos, sin, rope_rows, B, T, H, D, 0, nullptr, 0, nullptr};
+    kv.run = run; kv.group = group;
+    return quantize_launch(q, HBQ_DTYPE_F16, B * T * H, D, fmt, out, HBQ_DTYPE_F16, nullptr, nullptr, (cudaStream_t)stream, &kv);
+}
+
+int hbq_quantize_head_rows(const void* x, int64_t B, int64_t H, int64_t run, int64_t D, int64_t T0, int64_t T,
+                           const hbq_format* fmt, void* out, void* stream)
+{
+    if (!fmt || B < 0 || H <= 0 || run < 0 || D <= 0 || T0 < 0 || T0 + run > T || T > 0x7FFFFFFF) return HBQ_ERR_ARG;
+    if (B * run == 0) return HBQ_OK;
+    if (!out) return HBQ_ERR_ARG;
+    if (fmt->kind == HBQ_KIND_MXFP && fmt->per_tensor_scale) return HBQ_ERR_UNSUPPORTED;
+    KvWriteOpts kv = {nullptr, nullptr, 0, B, run, H, D, 0, nullptr, 0, nullptr};
+    kv.from_runs = 1; kv.T0 = T0; kv.Tall = T;
+    return quantize_launch(x, HBQ_DTYPE_F16, B * H * run, D, fmt, out, HBQ_DTYPE_F16, nullptr, nullptr, (cudaStream_t)stream, &kv);
+}
+
 int hbq_kv_write_v(const void* v, int dtype, int64_t B, int64_t T, int64_t H, int64_t D, const hbq_format* fmt,
                    void* out, int out_dtype, int out_token_major, void* stream)
 {

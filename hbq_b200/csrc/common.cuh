@@ -26,6 +26,9 @@ struct KvWriteOpts {
     int v_out_token_major;    // V only: write [B,T,H,D] instead of [B,H,T,D]
     const void* glu_gate;     // not a cache write: quantise silu(glu_gate) * x (fp16, same shape as x); the
                               // other fields are then unused
+    int64_t run = 0, group = 0;          // hbq_quantize_q_runs
+    int from_runs = 0;                   // hbq_quantize_head_rows
+    int64_t T0 = 0, Tall = 0;
 };
 
 #define HBQ_CUDA_TRY(expr)                                                     \

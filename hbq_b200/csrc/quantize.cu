@@ -857,11 +857,13 @@ int quantize_launch(const void* x, int dtype, int64_t rows, int64_t K, const hbq
         if (!deq) return HBQ_ERR_ARG;
         a.rope_cos = (const uint16_t*)kv->cos; a.rope_sin = (const uint16_t*)kv->sin; a.rope_rows = kv->rope_rows;
         a.perm_T = kv->T; a.perm_H = kv->H;
+        a.run = kv->run; a.group = kv->group; a.from_runs = kv->from_runs; a.T0 = kv->T0; a.Tall = kv->Tall;
         a.k_center = (const uint16_t*)kv->center;
         if (kv->center && ((reinterpret_cast<uintptr_t>(kv->center) & 15) || dtype != HBQ_DTYPE_F16 || kv->v_axis)) return HBQ_ERR_UNSUPPORTED;
         if ((kv->cos && ((reinterpret_cast<uintptr_t>(kv->cos) | reinterpret_cast<uintptr_t>(kv->sin)) & 15)) || !a.aligned)
             return HBQ_ERR_ALIGN;
     }
+    if (kv && (kv->run || kv->from_runs) && f->kind != HBQ_KIND_HBQ) return HBQ_ERR_UNSUPPORTED;
     if (f->kind == HBQ_KIND_MXEX || f->kind == HBQ_KIND_VSQ) {
         if (kv) return HBQ_ERR_UNSUPPORTED;
         return quantize_extra_launch(a, stream);
@@ -978,6 +980,7 @@ int quantize_launch(const void* x, int dtype, int64_t rows, int64_t K, const hbq
         bool launched = false;
         int rc = hbq_tab_try_launch(a, fast_mb, stream, &launched);          // byte-table kernels (quantize_tab.cu)
         if (rc != HBQ_OK || launched) return rc;
+        if (a.run || a.from_runs) return HBQ_ERR_UNSUPPORTED;                // row orders of the byte-table kernel only
         rc = hbq_lut_try_launch(a, fast_mb, stream, &launched);
         if (rc != HBQ_OK || launched) return rc;
     }

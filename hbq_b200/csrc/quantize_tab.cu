@@ -67,6 +67,9 @@ struct TabArgs {
     const uint4* rope_sin;
     const uint4* center;      // fp16 [B, H, block] or NULL: subtracted after the rotation
     uint32_t kv_T, kv_H, rope_rows;
+    uint32_t kv_B, run, group;    // run > 0: stored run by run of `run` tokens, the `group` heads of a key-value head together
+    uint32_t from_runs, T0;   // from_runs: the rows are (b, h, t), t the kv_T tokens of a run that starts at token T0,
+    uint32_t Tall;            // and stored at (b, T0 + t, h) of Tall tokens
     TabSecond b;              // hbq_tab_mix_kernel
 };
 static_assert(sizeof(TabArgs) <= 4000, "kernel parameters are limited to 4 KB");
@@ -478,9 +481,19 @@ __global__ void __launch_bounds__(TAB_THREADS, 2) hbq_tab_kernel(const TabArgs a
         int64_t o0 = c0;                                        // where chunk 0 is stored
         if (KV) {
             const uint32_t row = valid ? (uint32_t)bi : 0u;
-            const uint32_t bt = row / a.kv_H, h = row - bt * a.kv_H, b = bt / a.kv_T, t = bt - b * a.kv_T;
-            kv_rows<C>(a, rope_cos, rope_sin, center, xb, bt, b, t, h, Gt, g);
-            o0 = (((int64_t)b * a.kv_H + h) * a.kv_T + t) * (C * Gt) + g;
+            int64_t orow;
+            if (a.from_runs) {
+                const uint32_t bh = row / a.kv_T, t = row - bh * a.kv_T, b = bh / a.kv_H, h = bh - b * a.kv_H;
+                orow = ((int64_t)b * a.Tall + a.T0 + t) * a.kv_H + h;
+            } else {
+                const uint32_t bt = row / a.kv_H, h = row - bt * a.kv_H, b = bt / a.kv_T, t = bt - b * a.kv_T;
+                kv_rows<C>(a, rope_cos, rope_sin, center, xb, bt, b, t, h, Gt, g);
+                if (a.run) {
+                    const uint32_t hk = h / a.group, hg = h - hk * a.group, c = t / a.run, tc = t - c * a.run;
+                    orow = ((((int64_t)c * a.kv_B + b) * (a.kv_H / a.group) + hk) * a.group + hg) * a.run + tc;
+                } else orow = ((int64_t)b * a.kv_H + h) * a.kv_T + t;
+            }
+            o0 = orow * (C * Gt) + g;
         }
 
         // ---- block maximum and the E5M3 shared scale (round-half-up of the 3-bit mantissa) ----
@@ -1495,6 +1508,9 @@ int hbq_tab_try_launch(const QArgs& q, int mb, cudaStream_t stream, bool* launch
         a.rope_cos = reinterpret_cast<const uint4*>(q.rope_cos); a.rope_sin = reinterpret_cast<const uint4*>(q.rope_sin);
         a.center = reinterpret_cast<const uint4*>(q.k_center);
         a.kv_T = (uint32_t)q.perm_T; a.kv_H = (uint32_t)q.perm_H; a.rope_rows = (uint32_t)q.rope_rows;
+        a.kv_B = (uint32_t)(q.rows / (q.perm_T * q.perm_H));
+        a.run = (uint32_t)q.run; a.group = (uint32_t)q.group;
+        a.from_runs = (uint32_t)q.from_runs; a.T0 = (uint32_t)q.T0; a.Tall = (uint32_t)q.Tall;
     }
 
     const size_t smem = (size_t)(a.entries + (mix ? a.b.entries : 0)) * 4;

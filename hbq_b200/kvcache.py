@@ -127,6 +127,53 @@ def write_v_cache(v: torch.Tensor, num_heads: int, quantizer: _CudaBlockQuantize
     return out
 
 
+def _head_blocks(quantizer, D: int):
+    """The quantizer's format when it is an HBQ format whose block is one head's D values, else None."""
+    if not isinstance(quantizer, _CudaBlockQuantizer) or quantizer.out_dtype not in (None, torch.float16) or \
+            getattr(quantizer, "keep_l2_scale", False):
+        return None
+    f = quantizer._format()
+    return f if f.kind == _lib.KIND_HBQ and f.block_size == D else None
+
+
+def quantize_q_runs(q: torch.Tensor, num_heads: int, group: int, run: int, quantizer, cos: torch.Tensor,
+                    sin: torch.Tensor) -> Optional[torch.Tensor]:
+    """``write_k_cache`` of the post-RoPE queries, stored run by run: ``[T / run, B, H / group, group * run, D]``, each run
+    the left operand of its score product without a copy.  None where ``hbq_quantize_q_runs`` does not take the call."""
+    B, T = q.shape[0], q.shape[1]
+    D = _head_dim(q, num_heads)
+    fmt = _head_blocks(quantizer, D)
+    if fmt is None or q.dtype != torch.float16 or cos.dtype != torch.float16 or sin.dtype != torch.float16 or T % run or num_heads % group:
+        return None
+    qc = q.contiguous()
+    cos, sin, rope_rows = _tables(cos, sin, B, T, D)
+    out = torch.empty((T // run, B, num_heads // group, group * run, D), dtype=q.dtype, device=q.device)
+    with _lib.device_guard(q.device):
+        rc = _lib.lib().hbq_quantize_q_runs(_ptr(qc), B, T, num_heads, D, run, group, _ptr(cos), _ptr(sin), rope_rows,
+                                            ctypes.byref(fmt), _ptr(out), _stream_ptr(q.device))
+    if rc in (_lib.ERR_UNSUPPORTED, _lib.ERR_ALIGN):
+        return None
+    _lib.check(rc, "hbq_quantize_q_runs")
+    return out
+
+
+def quantize_head_rows(x: torch.Tensor, out: torch.Tensor, t0: int, quantizer) -> bool:
+    """``out[:, t0:t0 + run] = quantizer.q(x.transpose(1, 2))`` for a run's attention output ``x [B, H, run, D]`` and
+    ``out [B, T, H, D]`` with blocks of one head's D values; False (and nothing written) where
+    ``hbq_quantize_head_rows`` does not take the call."""
+    B, H, run, D = x.shape
+    fmt = _head_blocks(quantizer, D)
+    if fmt is None or x.dtype != torch.float16 or not x.is_contiguous():
+        return False
+    with _lib.device_guard(x.device):
+        rc = _lib.lib().hbq_quantize_head_rows(_ptr(x), B, H, run, D, t0, out.shape[1], ctypes.byref(fmt), _ptr(out),
+                                               _stream_ptr(x.device))
+    if rc in (_lib.ERR_UNSUPPORTED, _lib.ERR_ALIGN):
+        return False
+    _lib.check(rc, "hbq_quantize_head_rows")
+    return True
+
+
 FUSE_SWIGLU = True      # False: always run the separate ops (for A/B timing)
 
 

@@ -73,6 +73,10 @@ def rope_tables(T: int, head_dim: int, theta: float, device, offset: int = 0):
     return emb.cos().to(torch.float16)[None], emb.sin().to(torch.float16)[None]
 
 
+def _hooked(m: nn.Module) -> bool:
+    return bool(m._forward_hooks or m._forward_pre_hooks or "forward" in m.__dict__ or "q" in m.__dict__)
+
+
 def _same_format(a, b) -> bool:
     if type(a) is not type(b):
         return False
@@ -135,8 +139,16 @@ class QLlamaAttention(nn.Module):
         q = project(self.q_proj, x, input_quantized).view(bsz, q_len, H * D)
         k = project(self.k_proj, x, input_quantized).view(bsz, q_len, Hkv * D)
         v = project(self.v_proj, x, input_quantized).view(bsz, q_len, Hkv * D)
-        # RoPE, then the post-RoPE Q / K quantizers (src/module.py:158-162), in the cache layout [B, H, T, D]
-        if self.quant_post_rope_q and isinstance(self.q_proj.aq, _CudaBlockQuantizer):
+        # RoPE, then the post-RoPE Q / K quantizers (src/module.py:158-162), in the cache layout [B, H, T, D] -- the
+        # queries of a prefill that runs in pieces (below) piece by piece
+        c = self.query_chunk
+        in_runs = q_len > c and q_len % c == 0 and c % 128 == 0
+        Q = Qr = None
+        if in_runs and self.quant_post_rope_q and not _hooked(self.q_proj.aq):
+            Qr = kvcache.quantize_q_runs(q, H, G, c, self.q_proj.aq, cos, sin)
+        if Qr is not None:
+            pass
+        elif self.quant_post_rope_q and isinstance(self.q_proj.aq, _CudaBlockQuantizer):
             Q = kvcache.write_k_cache(q, H, self.q_proj.aq, cos, sin)
         else:
             Q = kvcache.apply_rope(q.view(bsz, q_len, H, D).transpose(1, 2), cos, sin)
@@ -158,24 +170,31 @@ class QLlamaAttention(nn.Module):
         # (1 - 1/runs) / 2 of both matmuls and of the softmax sweep.
         aq = self.attn_wgt_quantizer if self.quant_attn_wgt else None
         scale = 1.0 / math.sqrt(D)
-        c = self.query_chunk
-        if q_len <= c or q_len % c or c % 128:
+        if not in_runs:
             Qg = Q.contiguous().view(bsz, Hkv, G * q_len, D)
             scores = torch.matmul(Qg, K.transpose(-1, -2))                  # [B, Hkv, G*T, S] raw q k^T
             P = softmax_quantize(scores, scale, aq, causal=q_len > 1, q_len=q_len, heads=H)
             O = torch.matmul(P, V)                                          # [B, Hkv, G*T, D]
             O = O.view(bsz, H, q_len, D).transpose(1, 2).reshape(bsz * q_len, H * D)
         else:
-            Q5 = Q.contiguous().view(bsz, Hkv, G, q_len, D)
-            O4 = torch.empty((bsz, q_len, H, D), dtype=Q.dtype, device=Q.device)
+            Q5 = Q.contiguous().view(bsz, Hkv, G, q_len, D) if Qr is None else None
+            O4 = torch.empty((bsz, q_len, H, D), dtype=q.dtype, device=q.device)
+            # o_proj's input quantizer, where its blocks are heads, runs on each run's output while it is put in place
+            oq = self.o_proj.aq if not _hooked(self.o_proj.aq) else None
             for t0 in range(0, q_len, c):
                 t1 = t0 + c
-                Qc = Q5[:, :, :, t0:t1].reshape(bsz, Hkv, G * c, D)
+                Qc = Q5[:, :, :, t0:t1].reshape(bsz, Hkv, G * c, D) if Qr is None else Qr[t0 // c]
                 scores = torch.matmul(Qc, K[:, :, :t1].transpose(-1, -2))   # [B, Hkv, G*c, t1]
                 P = softmax_quantize(scores, scale, aq, causal=True, q_len=c, heads=H)
                 Oc = torch.matmul(P, V[:, :, :t1])                          # [B, Hkv, G*c, D]
-                O4[:, t0:t1] = Oc.view(bsz, H, c, D).transpose(1, 2)
+                Oc = Oc.view(bsz, H, c, D)
+                if oq is not None and not kvcache.quantize_head_rows(Oc, O4, t0, oq):
+                    oq = None                                               # refused at the first run or at none
+                if oq is None:
+                    O4[:, t0:t1] = Oc.transpose(1, 2)
             O = O4.view(bsz * q_len, H * D)
+            if oq is not None:
+                return project(self.o_proj, O, input_quantized=True)
         return project(self.o_proj, O)
 
 

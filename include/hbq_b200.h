@@ -123,6 +123,18 @@ int hbq_kv_write_k(const void* k, int dtype, int64_t B, int64_t T, int64_t H, in
                    const void* cos, const void* sin, int64_t rope_rows, const void* center,
                    const hbq_format* fmt, void* out, int out_dtype, void* stream);
 
+/* The query side of a prefill that is cut into runs of `run` queries (D = block size; fp16; formats of the byte-table
+ * kernel, else HBQ_ERR_UNSUPPORTED):
+ *   hbq_quantize_q_runs     hbq_kv_write_k with the output stored [T / run, B, H / group, group, run, D], so that a run is one
+ *                           dense batch of matrices.
+ *   hbq_quantize_head_rows  x [B, H, run, D] (a run's attention output) quantised along D and stored at tokens
+ *                           T0 .. T0 + run - 1 of out [B, T, H, D]: what quantising the transposed tensor's rows of H * D
+ *                           in blocks of D gives. */
+int hbq_quantize_q_runs(const void* q, int64_t B, int64_t T, int64_t H, int64_t D, int64_t run, int64_t group,
+                        const void* cos, const void* sin, int64_t rope_rows, const hbq_format* fmt, void* out, void* stream);
+int hbq_quantize_head_rows(const void* x, int64_t B, int64_t H, int64_t run, int64_t D, int64_t T0, int64_t T,
+                           const hbq_format* fmt, void* out, void* stream);
+
 /* V-cache write (src/module.py:163-168): v is the v_proj output viewed [B,T,H,D]; blocks of
  * fmt->block_size consecutive TOKENS per (batch, head, channel) are quantised (the tail block
  * zero padded) and the result is stored as [B,H,T,D] -- the reference's transpose, quantise,

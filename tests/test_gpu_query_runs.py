@@ -1,0 +1,61 @@
+"""GPU: the query side of a prefill in runs -- post-RoPE queries stored run by run, a run's attention output quantised into
+place -- against the plain quantizer on the same tensors permuted by torch, bit for bit; formats whose block is not one
+head are refused."""
+import pytest
+
+torch = pytest.importorskip("torch")
+pytestmark = pytest.mark.gpu
+
+
+def _quantizer(block, mb, micro):
+    import hbq_b200 as H
+    return H.HBQQuantizer(block, 2, mb, 5, 3, l2_block_size=micro, l2_sc_bit=2, l2_scheme="SIG-1")
+
+
+def _data(shape, seed):
+    g = torch.Generator(device="cuda").manual_seed(seed)
+    x = torch.randn(shape, device="cuda", generator=g)
+    x.view(-1, 32)[::5] *= 3000.0
+    x.view(-1, 32)[1::7] *= 1e-6
+    x.view(-1, 32)[2::9] = -0.0
+    return x.half()
+
+
+def _same(a, b):
+    return torch.equal(a.contiguous().view(torch.int16), b.contiguous().view(torch.int16))
+
+
+@pytest.mark.parametrize("D,mb,micro", [(128, 2, 8), (128, 1, 32), (64, 2, 8)])
+@pytest.mark.parametrize("B,T,heads,group,run", [(1, 256, 4, 1, 128), (2, 384, 6, 3, 128), (3, 24, 8, 8, 8), (1, 7, 2, 2, 7)])
+def test_q_runs(D, mb, micro, B, T, heads, group, run):
+    from hbq_b200 import kvcache
+    q, x = _quantizer(D, mb, micro), _data((B, T, heads * D), T + D)
+    ang = torch.rand((B, T, D), device="cuda", generator=torch.Generator(device="cuda").manual_seed(D)) * 6.28
+    for cos, sin in ((ang.cos().half(), ang.sin().half()), (ang[:1].cos().half(), ang[:1].sin().half())):
+        got = kvcache.quantize_q_runs(x, heads, group, run, q, cos, sin)
+        want = kvcache.write_k_cache(x, heads, q, cos, sin).view(B, heads // group, group, T // run, run, D).permute(3, 0, 1, 2, 4, 5)
+        assert _same(got, want.reshape(T // run, B, heads // group, group * run, D))
+
+
+@pytest.mark.parametrize("D,mb,micro", [(128, 2, 8), (128, 2, 32), (64, 1, 8)])
+@pytest.mark.parametrize("B,heads,run,t0,T", [(1, 1, 1, 0, 1), (2, 6, 128, 128, 384), (3, 5, 33, 10, 50)])
+def test_head_rows(D, mb, micro, B, heads, run, t0, T):
+    from hbq_b200 import kvcache
+    q, x = _quantizer(D, mb, micro), _data((B, heads, run, D), T + D)
+    out = torch.full((B, T, heads, D), 7.0, device="cuda", dtype=torch.float16)
+    want = out.clone()
+    assert kvcache.quantize_head_rows(x, out, t0, q)
+    want[:, t0:t0 + run] = q.q(x.transpose(1, 2).reshape(B * run, heads * D)).view(B, run, heads, D)
+    assert _same(out, want)
+
+
+def test_formats_that_are_refused():
+    import hbq_b200 as H
+    from hbq_b200 import kvcache
+    x, out = _data((1, 2, 16, 128), 1), torch.zeros((1, 16, 2, 128), device="cuda", dtype=torch.float16)
+    cos = torch.ones((1, 16, 128), device="cuda", dtype=torch.float16)
+    for q in (_quantizer(64, 2, 8), _quantizer(128, 3, 8), H.MXFPQuantizer(32, 2, 1, 5, 3), H.MXFPQuantizer(128, 2, 1, 5, 3),
+              H.HBQQuantizer(128, 2, 1, 5, 3, l2_block_size=8, l2_sc_bit=2, l2_scheme="Mix")):
+        assert not kvcache.quantize_head_rows(x, out, 0, q)
+        assert kvcache.quantize_q_runs(x.view(1, 16, 256), 2, 1, 8, q, cos, cos) is None
+    assert not out.any()
