@@ -27,7 +27,7 @@ EXPORTS = [
     "hbq_gemm", "hbq_gemm_workspace_bytes", "hbq_gemm_uses_tensor_cores", "hbq_gemm_simt",
     "hbq_gemm_kn_noalloc", "hbq_gemm_w4", "hbq_gemm_w4_prepack", "hbq_gemm_w4_prepacked_bytes",
     "hbq_gemm_w4_workspace_bytes", "hbq_kv_write_k", "hbq_kv_write_v", "hbq_swiglu_quantize", "hbq_rmsnorm_quantize", "hbq_softmax_quantize",
-    "hbq_quantize_q_runs", "hbq_quantize_head_rows", "hbq_moe_route", "hbq_gemm_grouped", "hbq_moe_combine",
+    "hbq_rope_heads", "hbq_quantize_q_runs", "hbq_quantize_head_rows", "hbq_moe_route", "hbq_gemm_grouped", "hbq_moe_combine",
     "hbq_gemm_status", "hbq_gemm_status_reset", "hbq_gemm_wait_selftest", "hbq_gemm_reserve_sms", "hbq_error_string", "hbq_last_cuda_error",
     "hbq_version", "hbq_launch_count",
 ]
@@ -87,6 +87,7 @@ def lib() -> ctypes.CDLL:
     L.hbq_gemm_w4_workspace_bytes.argtypes = [i64, i64, i64]
     L.hbq_gemm_w4_workspace_bytes.restype = i64
     L.hbq_gemm_w4.argtypes = [vp, vp, vp, i64, i64, i64, ctypes.POINTER(Format), ci, vp, vp, i64, vp]
+    L.hbq_rope_heads.argtypes = [vp, i64, i64, i64, i64, vp, vp, i64, vp, vp]
     L.hbq_quantize_q_runs.argtypes = [vp, i64, i64, i64, i64, i64, i64, vp, vp, i64, ctypes.POINTER(Format), vp, vp]
     L.hbq_quantize_head_rows.argtypes = [vp, i64, i64, i64, i64, i64, i64, ctypes.POINTER(Format), vp, vp]
     L.hbq_moe_route.argtypes = [vp, i64, ci, ci, vp, vp, vp, vp]

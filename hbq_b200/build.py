@@ -20,7 +20,7 @@ LIB_DIR = os.path.join(HERE, "lib")
 LIB_PATH = os.path.join(LIB_DIR, "libhbq_b200.so")
 HOST_PATH = os.path.join(LIB_DIR, "hbq_host.so")
 HOST_SOURCE = os.path.join(CSRC, "host.cpp")
-SOURCES = ["api.cu", "quantize.cu", "quantize_lut.cu", "quantize_tab.cu", "quantize_extra.cu", "dequantize.cu", "gemm_simt.cu", "gemm_tc.cu", "gemm_packed.cu", "gemm_static.cu", "moe.cu"]
+SOURCES = ["api.cu", "quantize.cu", "quantize_lut.cu", "quantize_tab.cu", "quantize_extra.cu", "dequantize.cu", "gemm_simt.cu", "gemm_tc.cu", "gemm_packed.cu", "gemm_static.cu", "moe.cu", "rope.cu"]
 HEADERS = [os.path.join(CSRC, "common.cuh"), os.path.join(CSRC, "quantize_dev.cuh"), os.path.join(CSRC, "vcache_dev.cuh"), os.path.join(CSRC, "quantize_tab.cuh"), os.path.join(CSRC, "tc_dev.cuh"), os.path.join(HERE, "..", "include", "hbq_b200.h")]
 NVCC_FLAGS = ["-gencode", "arch=compute_100a,code=sm_100a", "-lineinfo", "-O3", "-std=c++17",
               "-Xcompiler", "-fPIC", "-shared", "--threads", "4"]

@@ -88,6 +88,7 @@ int gemm_tc_grouped_launch(const void*, int64_t, const int*, int, const void* co
                            int, int, cudaStream_t);
 int moe_route_launch(const int64_t*, int64_t, int, int, int*, int64_t*, int*, cudaStream_t);                      // moe.cu
 int moe_combine_launch(const void*, const void*, const int*, int64_t, int, int64_t, void*, cudaStream_t);
+int rope_heads_launch(const void*, int64_t, int64_t, int64_t, int64_t, const void*, const void*, int64_t, void*, cudaStream_t);   // rope.cu
 int64_t gemm_w4_prepacked_bytes(int64_t, int64_t, int);
 int gemm_w4_prepack(const hbq_packed_out*, int64_t, int64_t, const hbq_format*, int, void*, cudaStream_t);
 int64_t gemm_w4_workspace_bytes(int64_t, int64_t, int64_t);
@@ -118,6 +119,12 @@ int hbq_kv_write_k(const void* k, int dtype, int64_t B, int64_t T, int64_t H, in
     if (fmt->kind == HBQ_KIND_MXFP && fmt->per_tensor_scale) return HBQ_ERR_UNSUPPORTED;   // needs max|x| of the rotated tensor first
     KvWriteOpts kv = {cos, sin, rope_rows, B, T, H, D, 0, center, 0, nullptr};
     return quantize_launch(k, dtype, B * T * H, D, fmt, out, out_dtype, nullptr, nullptr, (cudaStream_t)stream, &kv);
+}
+
+int hbq_rope_heads(const void* x, int64_t B, int64_t T, int64_t H, int64_t D, const void* cos, const void* sin, int64_t rope_rows,
+                   void* out, void* stream)
+{
+    return rope_heads_launch(x, B, T, H, D, cos, sin, rope_rows, out, (cudaStream_t)stream);
 }
 
 int hbq_quantize_q_runs(const void* q, int64_t B, int64_t T, int64_t H, int64_t D, int64_t run, int64_t group, const void* cos,

@@ -33,6 +33,25 @@ def apply_rope(x: torch.Tensor, cos: torch.Tensor, sin: torch.Tensor) -> torch.T
     return (x * cos) + (rotate_half(x) * sin)
 
 
+def rope_heads(x: torch.Tensor, num_heads: int, cos: torch.Tensor, sin: torch.Tensor) -> torch.Tensor:
+    """``apply_rope(x.view(B, T, H, D).transpose(1, 2), cos, sin)`` for a projection output ``x [B, T, H * D]``, in one pass
+    where ``hbq_rope_heads`` takes it (fp16 CUDA tensors without a gradient to record), else the separate ops."""
+    B, T = x.shape[0], x.shape[1]
+    D = _head_dim(x, num_heads)
+    if x.is_cuda and x.dtype == torch.float16 and cos.dtype == torch.float16 and sin.dtype == torch.float16 and \
+            cos.device == x.device and sin.device == x.device and cos.dim() == 3 and \
+            not (torch.is_grad_enabled() and (x.requires_grad or cos.requires_grad or sin.requires_grad)):
+        xc = x.contiguous()
+        c, s, rope_rows = _tables(cos, sin, B, T, D)
+        out = torch.empty((B, num_heads, T, D), dtype=x.dtype, device=x.device)
+        with _lib.device_guard(x.device):
+            rc = _lib.lib().hbq_rope_heads(_ptr(xc), B, T, num_heads, D, _ptr(c), _ptr(s), rope_rows, _ptr(out), _stream_ptr(x.device))
+        if rc not in (_lib.ERR_UNSUPPORTED, _lib.ERR_ALIGN):
+            _lib.check(rc, "hbq_rope_heads")
+            return out
+    return apply_rope(x.reshape(B, T, num_heads, D).transpose(1, 2), cos, sin)
+
+
 def _head_dim(x: torch.Tensor, num_heads: int) -> int:
     if x.dim() == 4 and x.shape[2] == num_heads:
         return x.shape[3]

@@ -151,13 +151,13 @@ class QLlamaAttention(nn.Module):
         elif self.quant_post_rope_q and isinstance(self.q_proj.aq, _CudaBlockQuantizer):
             Q = kvcache.write_k_cache(q, H, self.q_proj.aq, cos, sin)
         else:
-            Q = kvcache.apply_rope(q.view(bsz, q_len, H, D).transpose(1, 2), cos, sin)
+            Q = kvcache.rope_heads(q, H, cos, sin)
             if self.quant_post_rope_q:
                 Q = self.q_proj.aq.q(Q)
         if self.quant_k_cache and isinstance(self.kv_quantizer, _CudaBlockQuantizer):
             K = kvcache.write_k_cache(k, Hkv, self.kv_quantizer, cos, sin)
         else:
-            K = kvcache.apply_rope(k.view(bsz, q_len, Hkv, D).transpose(1, 2), cos, sin)
+            K = kvcache.rope_heads(k, Hkv, cos, sin)
         # V quantised along the token axis (src/module.py:163-168)
         if self.quant_v_cache and isinstance(self.kv_quantizer, _CudaBlockQuantizer):
             V = kvcache.write_v_cache(v, Hkv, self.kv_quantizer)

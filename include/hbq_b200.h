@@ -123,6 +123,10 @@ int hbq_kv_write_k(const void* k, int dtype, int64_t B, int64_t T, int64_t H, in
                    const void* cos, const void* sin, int64_t rope_rows, const void* center,
                    const hbq_format* fmt, void* out, int out_dtype, void* stream);
 
+/* hbq_kv_write_k without the quantizer: x [B, T, H, D] fp16 rotated and stored [B, H, T, D]. */
+int hbq_rope_heads(const void* x, int64_t B, int64_t T, int64_t H, int64_t D, const void* cos, const void* sin,
+                   int64_t rope_rows, void* out, void* stream);
+
 /* The query side of a prefill that is cut into runs of `run` queries (D = block size; fp16; formats of the byte-table
  * kernel, else HBQ_ERR_UNSUPPORTED):
  *   hbq_quantize_q_runs     hbq_kv_write_k with the output stored [T / run, B, H / group, group, run, D], so that a run is one
