@@ -10,26 +10,32 @@ constexpr int ROUTE_MAX_EXPERTS = 256;
 
 // A stable counting sort of n expert ids by ONE CTA: warp w owns a contiguous run of the copies, counts them per expert
 // (lanes with the same id find each other with match.any), the counts become start positions in (expert, warp) order,
-// and the second sweep hands them out.  2000 copies of 8 experts: 4.0 us (the radix sort
+// and the second sweep hands them out.  An id outside [0, experts) counts as one of a further, last bucket: its copies
+// lie behind every expert's rows and have no position (pos -1).  2000 copies of 8 experts: 4.0 us (the radix sort
 // alone took 25, before its histogram, division and a host synchronisation).
 __global__ void __launch_bounds__(ROUTE_WARPS * 32) moe_route_kernel(const int64_t* ids, int n, int top_k, int experts,
                                                                       int* offsets, int64_t* src_rows, int* pos)
 {
-    __shared__ int s_cnt[ROUTE_MAX_EXPERTS][ROUTE_WARPS + 1];
-    __shared__ int s_off[ROUTE_MAX_EXPERTS + 1];
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    for (int i = threadIdx.x; i < experts * (ROUTE_WARPS + 1); i += ROUTE_WARPS * 32) (&s_cnt[0][0])[i] = 0;
+    __shared__ int s_cnt[ROUTE_MAX_EXPERTS + 1][ROUTE_WARPS + 1];
+    __shared__ int s_off[ROUTE_MAX_EXPERTS + 2];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, buckets = experts + 1;
+    for (int i = threadIdx.x; i < buckets * (ROUTE_WARPS + 1); i += ROUTE_WARPS * 32) (&s_cnt[0][0])[i] = 0;
     __syncthreads();
     const int run = (n + ROUTE_WARPS * 32 - 1) / (ROUTE_WARPS * 32) * 32;
     const int c0 = warp * run, c1 = min(c0 + run, n);
+    auto bucket = [&](int c) -> int {                            // -1: no copy; compared in 64 bits, before it is narrowed
+        if (c >= c1) return -1;
+        const int64_t id = ids[c];
+        return id >= 0 && id < experts ? (int)id : experts;
+    };
     for (int c = c0; c < c1; c += 32) {
-        const int e = c + lane < c1 ? (int)ids[c + lane] : -1;
+        const int e = bucket(c + lane);
         const uint32_t same = __match_any_sync(0xFFFFFFFFu, e);
         if (e >= 0 && lane == __ffs(same) - 1) s_cnt[e][warp] += __popc(same);
         __syncwarp();
     }
     __syncthreads();
-    for (int e = warp; e < experts; e += ROUTE_WARPS) {          // a warp per expert: prefix sum over the warps' counts
+    for (int e = warp; e < buckets; e += ROUTE_WARPS) {          // a warp per bucket: prefix sum over the warps' counts
         const int v = s_cnt[e][lane];
         int inc = v;
         #pragma unroll
@@ -43,12 +49,12 @@ __global__ void __launch_bounds__(ROUTE_WARPS * 32) moe_route_kernel(const int64
     __syncthreads();
     if (threadIdx.x == 0) {
         s_off[0] = 0;
-        for (int e = 0; e < experts; ++e) s_off[e + 1] += s_off[e];
+        for (int e = 0; e < buckets; ++e) s_off[e + 1] += s_off[e];
     }
     __syncthreads();
     for (int e = threadIdx.x; e <= experts; e += ROUTE_WARPS * 32) offsets[e] = s_off[e];
     for (int c = c0; c < c1; c += 32) {
-        const int e = c + lane < c1 ? (int)ids[c + lane] : -1;
+        const int e = bucket(c + lane);
         const uint32_t same = __match_any_sync(0xFFFFFFFFu, e);
         int base = 0;
         if (e >= 0) base = s_cnt[e][warp];
@@ -56,7 +62,7 @@ __global__ void __launch_bounds__(ROUTE_WARPS * 32) moe_route_kernel(const int64
         if (e >= 0) {
             const int p = s_off[e] + base + __popc(same & ((1u << lane) - 1u));
             src_rows[p] = (c + lane) / top_k;
-            pos[c + lane] = p;
+            pos[c + lane] = e < experts ? p : -1;
             if (lane == __ffs(same) - 1) s_cnt[e][warp] = base + __popc(same);
         }
         __syncwarp();
@@ -76,7 +82,9 @@ __global__ void __launch_bounds__(256) moe_combine_kernel(const uint4* __restric
         float acc[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
         for (int j = 0; j < top_k; ++j) {
             const int64_t k = t * top_k + j;
-            const uint4 v = __ldg(rows + (int64_t)__ldg(pos + k) * cpr + c);
+            const int p0 = __ldg(pos + k);
+            if (p0 < 0) continue;                                // a copy without an expert
+            const uint4 v = __ldg(rows + (int64_t)p0 * cpr + c);
             const __half2 wv = __half2half2(w[k]);
             const uint32_t r[4] = {v.x, v.y, v.z, v.w};
             #pragma unroll

@@ -256,10 +256,12 @@ int hbq_gemm_wait_selftest(const void* A, const void* W, void* C, int64_t M, int
  * MixtralSparseMoeBlock whose experts the reference patches, src/module.py:597-622), without a host read.
  *   hbq_moe_route    ids [tokens, top_k] (int64 expert of each copy) -> offsets [experts + 1], src_rows [tokens * top_k]
  *                    (token of each copy, copies stably sorted by expert), pos [tokens * top_k] (a copy's sorted row).
+ *                    A copy whose id is outside [0, experts) belongs to no expert: it is sorted behind offsets[experts]
+ *                    and its pos is -1.
  *   hbq_gemm_grouped entry i: C_host[i][r, :] = A[r, :] * W_host[i][N, K]^T for the rows of expert expert_host[i], i.e.
  *                    offsets[e] .. offsets[e + 1] - 1; A [rows, K], accumulation model as hbq_gemm (FP32, GROUPED,
  *                    PSUM_INT8 with group_n = 32).  W_host / C_host / expert_host are host arrays of `entries`.
- *   hbq_moe_combine  out[t, :] = sum_j fp16(y_rows[pos[t * top_k + j], :] * weights[t, j]). */
+ *   hbq_moe_combine  out[t, :] = sum_j fp16(y_rows[pos[t * top_k + j], :] * weights[t, j]) over the copies with pos >= 0. */
 int hbq_moe_route(const int64_t* ids, int64_t tokens, int top_k, int experts, int32_t* offsets, int64_t* src_rows,
                   int32_t* pos, void* stream);
 int hbq_gemm_grouped(const void* A, int64_t rows, const int32_t* offsets, int entries, const void* const* W_host,

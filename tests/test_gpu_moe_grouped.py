@@ -74,3 +74,40 @@ def test_route_is_a_stable_sort(E, tokens, top_k):
     assert torch.equal(pos.long()[order], torch.arange(tokens * top_k, device="cuda"))
     counts = torch.bincount(ids.view(-1), minlength=E)
     assert torch.equal(off.long(), torch.cat([counts.new_zeros(1), counts.cumsum(0)]))
+
+
+@pytest.mark.parametrize("E,tokens,top_k", [(1, 1, 1), (8, 33, 2), (33, 1000, 3), (256, 5000, 2)])
+def test_ids_without_an_expert_are_left_out(E, tokens, top_k):
+    """Ids below 0, of the number of experts and more, and beyond 32 bits: their copies lie behind every expert's rows,
+    have no position and add nothing to their token."""
+    from hbq_b200 import _lib
+    from hbq_b200.quantizer import _ptr, _stream_ptr
+    g = torch.Generator(device="cuda").manual_seed(E + tokens)
+    n = tokens * top_k
+    ids = torch.randint(0, E, (n,), device="cuda", generator=g)
+    odd = torch.tensor([-1, E, -2 ** 31, 2 ** 31, 2 ** 32, 2 ** 32 + E - 1, -2 ** 63, 2 ** 63 - 1], device="cuda")
+    hit = torch.rand(n, device="cuda", generator=g) < 0.3
+    hit[0] = True
+    ids = torch.where(hit, odd[torch.arange(n, device="cuda") % 8], ids)
+    valid = (ids >= 0) & (ids < E)
+    off = torch.empty(E + 1, dtype=torch.int32, device="cuda")
+    pos = torch.empty(n, dtype=torch.int32, device="cuda")
+    src = torch.empty(n, dtype=torch.int64, device="cuda")
+    s, L = _stream_ptr(ids.device), _lib.lib()
+    _lib.check(L.hbq_moe_route(_ptr(ids), tokens, top_k, E, _ptr(off), _ptr(src), _ptr(pos), s), "route")
+    order = torch.sort(torch.where(valid, ids, E), stable=True).indices
+    count = int(valid.sum())
+    assert torch.equal(src, order // top_k)
+    assert torch.equal(pos.long()[order], torch.where(torch.arange(n, device="cuda") < count, torch.arange(n, device="cuda"), -1))
+    counts = torch.bincount(ids[valid], minlength=E)
+    assert torch.equal(off.long(), torch.cat([counts.new_zeros(1), counts.cumsum(0)]))
+    hidden = 64
+    rows = torch.randn((n, hidden), device="cuda", generator=g).half()
+    w = torch.rand((tokens, top_k), device="cuda", generator=g).half()
+    out = torch.empty((tokens, hidden), dtype=torch.float16, device="cuda")
+    _lib.check(L.hbq_moe_combine(_ptr(rows), _ptr(w), _ptr(pos), tokens, top_k, hidden, _ptr(out), s), "combine")
+    parts = torch.where(valid[:, None], rows[pos.long().clamp(min=0)] * w.view(-1, 1), 0).view(tokens, top_k, hidden).float()
+    want = torch.zeros((tokens, hidden), device="cuda")
+    for j in range(top_k):                               # the kernel's order: fp32 sums of the fp16 products
+        want += parts[:, j]
+    assert torch.equal(out, want.half())
