@@ -221,7 +221,8 @@ class ExpertParallelMoE(nn.Module):
         x2d = x.reshape(-1, self.hidden)
         w, idx = self.route(x2d)
         model = self._grouped_model() if x2d.is_cuda and x2d.dtype == torch.float16 and x2d.shape[0] else None
-        if model is not None:
+        # (a `route` of the caller's own may return other types, which the kernels do not read)
+        if model is not None and idx.dtype == torch.int64 and w.dtype == torch.float16 and idx.shape == w.shape == (x2d.shape[0], self.top_k):
             return dict(self._begin_local(lead, x2d, w, idx), model=model)
         flat_e = idx.reshape(-1)                                       # expert of copy c = (token c // k, choice c % k)
         order = torch.sort(flat_e, stable=True).indices               # copies grouped by expert, hence by rank

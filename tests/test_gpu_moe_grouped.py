@@ -56,6 +56,24 @@ def test_grouped_experts_equal_one_at_a_time(ops, E, top_k, tokens):
     assert H.gemm_status() == 0
 
 
+def test_expert_ids_of_another_integer_type():
+    """A block with a router of its own that returns 32-bit ids: the same result as with 64-bit ones."""
+    import hbq_b200 as H
+
+    class Block(H.ExpertParallelMoE):
+        def route(self, x2d):
+            w, idx = super().route(x2d)
+            return w, idx.int()
+
+    moe = _block(8, 2, 256, 640, _ops("fp16"))
+    x = torch.randn((77, 256), device="cuda").half()
+    with torch.inference_mode():
+        want = moe(x)
+        moe.__class__ = Block
+        got = moe(x)
+    assert torch.equal(got.view(torch.int16), want.view(torch.int16))
+
+
 @pytest.mark.parametrize("E", [1, 2, 8, 33, 256])
 @pytest.mark.parametrize("tokens,top_k", [(1, 1), (31, 2), (512, 2), (1000, 3), (40000, 2)])
 def test_route_is_a_stable_sort(E, tokens, top_k):
