@@ -8,7 +8,8 @@
 // Element values without tables: exponent and mantissa of a code, put at the top of the mantissa and the bottom of
 // the exponent field of an fp16 pattern, are the value times 2^(bias - 15) -- subnormal codes included -- so one
 // exact multiply by 2^(15 - bias) decodes any format of up to five exponent bits; integers go through the pattern
-// of 1024 + v.
+// of 1024 + v.  With five exponent bits the top field stands for 2^16 and more, beyond fp16: infinity whatever the
+// mantissa says, so the mantissa is cleared there (its pattern would be a NaN's).
 // HBQ weight [14336, 4096] (150 MB moved): 37 us = 4.0 TB/s; one chunk per thread with scalar ldexpf decoding and a
 // 64-bit division each took 301 us.
 #include "quantize_dev.cuh"
@@ -33,6 +34,7 @@ struct DqArgs {
     uint32_t magmask2;        // FP codes: magnitude bits, in both halves
     int mshift, sshift;       // magnitude / sign -> their place in an fp16 pattern
     uint32_t unbias2;         // 2^(15 - bias) as an fp16 pair
+    int e5;                   // five exponent bits
     int log2L, l2_bits, l2_bytes, l2_aligned;
     uint32_t tab2[2][16];     // HBQ candidates as fp16 pairs
 };
@@ -48,7 +50,9 @@ __device__ __forceinline__ __half2 decode_pair(const DqArgs& a, uint32_t b, uint
         return __hsub2(bits_h2((b ^ FLIP) | 0x64006400u), bits_h2(0x64006400u | FLIP));
     }
     const uint32_t s = BITS == 5 ? ss : (b << a.sshift) & 0x80008000u;
-    return __hmul2(bits_h2(((b & a.magmask2) << a.mshift) | s), bits_h2(a.unbias2));
+    uint32_t v = (b & a.magmask2) << a.mshift;
+    if (BITS == 8 && a.e5) v = __vminu2(v, 0x7C007C00u);
+    return __hmul2(bits_h2(v | s), bits_h2(a.unbias2));
 }
 
 template <int BITS, bool INT, bool HBQ>
@@ -151,6 +155,7 @@ int dequantize_launch(const hbq_packed_out* in, int64_t rows, int64_t K, const h
         if (code_bits < 4) code_bits = 4;
         if (code_bits > 5) code_bits = 8;
         const int mag_bits = f->ebit + f->mbit;
+        a.e5 = f->ebit == 5;
         a.magmask2 = ((1u << mag_bits) - 1u) * 0x00010001u;
         a.mshift = 10 - f->mbit;
         a.sshift = 15 - (code_bits == 4 ? 3 : mag_bits);

@@ -33,3 +33,22 @@ def test_dequantize_equals_the_quantizers_tensor(name, rows, K, dtype):
         raw[1:] = packed.l2_packed.flatten()
         packed.l2_packed = raw[1:].view(packed.l2_packed.shape)
         assert torch.equal(H.dequantize_packed(packed).view(torch.int16), a)
+
+
+@pytest.mark.parametrize("mbit", [0, 1, 2])
+def test_codes_beyond_fp16_decode_to_infinity(mbit):
+    """Five exponent bits: every code times a scale of one, against the value sign * 2^(e - 15) * (1 + m) in 64 bits rounded
+    to fp16 -- the top exponent is 2^16 and more, infinite with any mantissa."""
+    import hbq_b200 as H
+    q = H.MXFPQuantizer(32, 5, mbit, 5, 3)
+    bits = 6 + mbit
+    packed = q.quantize_packed(torch.zeros((1 << bits, 32), device="cuda").half())
+    packed.codes = torch.arange(1 << bits, device="cuda", dtype=torch.uint8).view(-1, 1).expand(-1, 32).contiguous()
+    packed.scale_u8 = torch.full_like(packed.scale_u8, 0x3C00 >> 7)
+    c = torch.arange(1 << bits, dtype=torch.float64)
+    m, e = c % (1 << mbit), (c // (1 << mbit)) % 32
+    mag = torch.where(e == 0, m / (1 << mbit) * 2.0 ** -14, (1 + m / (1 << mbit)) * 2.0 ** (e - 15))
+    want = torch.where(c >= 1 << (5 + mbit), -mag, mag).half()
+    got = H.dequantize_packed(packed).cpu()
+    assert torch.isinf(want).sum() == 2 << mbit
+    assert torch.equal(got.view(torch.int16), want.view(-1, 1).expand(-1, 32).contiguous().view(torch.int16))
