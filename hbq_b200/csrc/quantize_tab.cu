@@ -611,9 +611,9 @@ __global__ void __launch_bounds__(TAB_THREADS, 2) hbq_tab_kernel(const TabArgs a
 // use (chunk distance 8, 4, 2, 1), so a sum that the fp32 additions round is the same number in all of them.
 // Bound: instruction issue (about twice hbq_tab_kernel's work per element).  Weight [14336, 4096] to packed planes:
 // 136 us; the arithmetic kernel of quantize.cu, which alone had these outputs, took 507 us.
-// INF: an infinite |x|, whose quotient comes out of the division as NaN, takes the largest level (the minimum drops the
-// NaN); otherwise it takes the smallest, as in the other kernels that form the tensor alone.
-template <int MB, int C, int ML, bool SMALL, bool INF>
+// An infinite |x|, whose quotient comes out of the division as NaN, takes the largest level: the minimum, which drops
+// the NaN, is the inner one.
+template <int MB, int C, int ML, bool SMALL>
 __device__ __forceinline__ void scheme_chunks(const uint32_t tab_addr, uint32_t base2, uint32_t hi2, uint32_t entry_bytes,
                                               const uint32_t* nt2, const uint32_t (*xb)[4], uint32_t l1b, const uint4 cst,
                                               int m_lanes, uint32_t& bests, uint32_t (*win)[2], float* err, uint32_t& amin)
@@ -636,8 +636,7 @@ __device__ __forceinline__ void scheme_chunks(const uint32_t tab_addr, uint32_t 
             const __half2 r = __hfma2(q0, nm2, axs);
             const __half2 aa = __hmul2(__hfma2(r, rm2, q0), post2);
             amin = h2_bits(__hmin2(bits_h2(amin), aa));
-            const uint32_t w = INF ? h2_bits(__hmax2(__hmin2(aa, bits_h2(hi2)), bits_h2(base2)))
-                                   : h2_bits(__hmin2(__hmax2(aa, bits_h2(base2)), bits_h2(hi2)));
+            const uint32_t w = h2_bits(__hmax2(__hmin2(aa, bits_h2(hi2)), bits_h2(base2)));
             asm volatile("ld.shared.u32 %0, [%1];" : "=r"(ent[2 * p]) : "r"((w & 0xFFFFu) * entry_bytes + addr0));
             asm volatile("ld.shared.u32 %0, [%1];" : "=r"(ent[2 * p + 1]) : "r"((w >> 16) * entry_bytes + addr0));
         }
@@ -666,9 +665,6 @@ __device__ __forceinline__ void scheme_chunks(const uint32_t tab_addr, uint32_t 
         win[k][1] = prmt(prmt(ent[4], ent[5], sel), prmt(ent[6], ent[7], sel), 0x5410u);
     }
 }
-
-template <bool KEEP_NAN>
-__device__ __forceinline__ __half2 block_max2(__half2 a, __half2 b) { return KEEP_NAN ? __hmax2_nan(a, b) : __hmax2(a, b); }
 
 template <int MB, int GT, int ML, bool SIDE>
 __global__ void __launch_bounds__(MIX_THREADS, 2) hbq_tab_mix_kernel(const TabArgs a)
@@ -708,18 +704,17 @@ __global__ void __launch_bounds__(MIX_THREADS, 2) hbq_tab_mix_kernel(const TabAr
                 for (int p = 0; p < 4; ++p)
                     xb[k][p] = h2_bits(__floats2half2_rn(__uint_as_float(xb[k][p] << 16), __uint_as_float(xb[k][p] & 0xFFFF0000u)));
         }
-        // The block maximum serves both schemes; their scales differ by the largest candidate.  With packed outputs it is
-        // taken with the maximum that keeps a NaN (the same cost), so that blocks with one are known; a NaN does not
-        // count for the scale.
+        // The block maximum serves both schemes; their scales differ by the largest candidate.  It is taken with the
+        // maximum that keeps a NaN (the same cost), so that blocks with one are known; a NaN does not count for the scale.
         uint32_t mx = 0u;
         #pragma unroll
         for (int k = 0; k < C; ++k)
             #pragma unroll
-            for (int p = 0; p < 4; ++p) mx = h2_bits(block_max2<SIDE>(bits_h2(mx), __habs2(bits_h2(xb[k][p]))));
+            for (int p = 0; p < 4; ++p) mx = h2_bits(__hmax2_nan(bits_h2(mx), __habs2(bits_h2(xb[k][p]))));
         for (int off = Gt >> 1; off >= 1; off >>= 1)
-            mx = h2_bits(block_max2<SIDE>(bits_h2(mx), bits_h2(__shfl_xor_sync(0xFFFFFFFFu, mx, off))));
-        const bool nans = SIDE && max(mx & 0x7FFFu, (mx >> 16) & 0x7FFFu) > 0x7C00u;
-        if (SIDE && __any_sync(0xFFFFFFFFu, nans)) {
+            mx = h2_bits(__hmax2_nan(bits_h2(mx), bits_h2(__shfl_xor_sync(0xFFFFFFFFu, mx, off))));
+        const bool nans = max(mx & 0x7FFFu, (mx >> 16) & 0x7FFFu) > 0x7C00u;
+        if (__any_sync(0xFFFFFFFFu, nans)) {
             mx = 0u;
             #pragma unroll
             for (int k = 0; k < C; ++k)
@@ -734,12 +729,12 @@ __global__ void __launch_bounds__(MIX_THREADS, 2) hbq_tab_mix_kernel(const TabAr
         uint32_t bests, bests1, win[C][2], win1[C][2], amin, amin1;
         float err[C], err1[C];
         const bool small = __all_sync(0xFFFFFFFFu, l1a < a.big_l1 && l1c < a.b.big_l1);
-        if (small) scheme_chunks<MB, C, ML, true, SIDE>(dst, a.base2, a.hi2, a.entry_bytes, a.nt2, xb, l1a, s_l1c[l1a >> 7], a.m_lanes, bests, win, err, amin);
-        else scheme_chunks<MB, C, ML, false, SIDE>(dst, a.base2, a.hi2, a.entry_bytes, a.nt2, xb, l1a, s_l1c[l1a >> 7], a.m_lanes, bests, win, err, amin);
+        if (small) scheme_chunks<MB, C, ML, true>(dst, a.base2, a.hi2, a.entry_bytes, a.nt2, xb, l1a, s_l1c[l1a >> 7], a.m_lanes, bests, win, err, amin);
+        else scheme_chunks<MB, C, ML, false>(dst, a.base2, a.hi2, a.entry_bytes, a.nt2, xb, l1a, s_l1c[l1a >> 7], a.m_lanes, bests, win, err, amin);
         const float tot = block_error<C>(err, Gt);
         const uint32_t dst1 = dst + (uint32_t)a.entries * 4u;
-        if (small) scheme_chunks<MB, C, ML, true, SIDE>(dst1, a.b.base2, a.b.hi2, a.entry_bytes, a.b.nt2, xb, l1c, s_l1c[l1c >> 7], a.m_lanes, bests1, win1, err1, amin1);
-        else scheme_chunks<MB, C, ML, false, SIDE>(dst1, a.b.base2, a.b.hi2, a.entry_bytes, a.b.nt2, xb, l1c, s_l1c[l1c >> 7], a.m_lanes, bests1, win1, err1, amin1);
+        if (small) scheme_chunks<MB, C, ML, true>(dst1, a.b.base2, a.b.hi2, a.entry_bytes, a.b.nt2, xb, l1c, s_l1c[l1c >> 7], a.m_lanes, bests1, win1, err1, amin1);
+        else scheme_chunks<MB, C, ML, false>(dst1, a.b.base2, a.b.hi2, a.entry_bytes, a.b.nt2, xb, l1c, s_l1c[l1c >> 7], a.m_lanes, bests1, win1, err1, amin1);
         const float tot1 = block_error<C>(err1, Gt);
         const bool second = rh(tot1) < rh(tot);                  // the same in every lane of the block
         if (second) {
@@ -783,7 +778,7 @@ __global__ void __launch_bounds__(MIX_THREADS, 2) hbq_tab_mix_kernel(const TabAr
                 const __half2 dneg = small ? __hmul2(bits_h2(cw[p]), tlb) : __hmul2(__hmul2(bits_h2(cw[p]), bits_h2(nt)), bits_h2(l1u));
                 dq[p] = (h2_bits(dneg) & 0x7FFF7FFFu) | sg[p];
             }
-            if (SIDE && nans) {                                  // a NaN stays one in the tensor; its code has all bits set (E2M2: no sign)
+            if (nans) {                                 // a NaN stays one in the tensor; its code has all bits set (E2M2: no sign)
                 #pragma unroll
                 for (int p = 0; p < 4; ++p)
                     #pragma unroll

@@ -79,3 +79,27 @@ def test_mix_packed_outputs_of_infinite_and_nan_inputs(oracle, block, micro, mb)
     assert np.array_equal(packed.scheme.cpu().numpy(), o["scheme"])
     got = deq.cpu().numpy()
     assert np.array_equal(bits(got)[ok], bits(o["deq"].reshape(41, -1))[ok]) and np.isnan(got[~ok]).all()
+
+
+@pytest.mark.parametrize("block,micro,mb", [(128, 8, 1), (128, 32, 2), (64, 16, 1), (32, 8, 1)])
+def test_mix_tensor_of_infinite_and_nan_inputs_does_not_depend_on_the_outputs(oracle, block, micro, mb):
+    """The tensor alone, with the kept scales and with packed outputs: the oracle's values, NaNs included."""
+    import hbq_b200 as H
+    x = _inputs(41, 1536, 7)
+    rng = np.random.default_rng(8)
+    x[rng.random(x.shape) < 0.004] = np.float16(np.inf)
+    x[rng.random(x.shape) < 0.004] = np.float16(-np.inf)
+    x[3, :block] = np.float16(-np.inf)
+    x[rng.random(x.shape) < 0.002] = np.float16(np.nan)
+    x[5, :block] = np.float16(np.nan)
+    ok = ~np.isnan(x)
+    want = oracle.quantize(x, oracle.Format(oracle.KIND_HBQ, 2, mb, 5, 3, block, l2_block_size=micro, l2_sc_bit=2, l2_scheme="Mix"))["deq"].reshape(41, -1)
+    assert np.isinf(want).any()
+    kw = dict(block_size=block, ebit=2, mbit=mb, sc_ebit=5, sc_mbit=3, l2_block_size=micro, l2_sc_bit=2, l2_scheme="Mix")
+    t = torch.from_numpy(x).cuda()
+    got = [H.HBQQuantizer(**kw).q(t), H.HBQQuantizer(keep_l2_scale=True, **kw).q(t)]
+    if (block // micro) * 2 in (8, 16, 32):
+        got.append(H.HBQQuantizer(**kw).quantize_packed(t, with_deq=True)[1])
+    for y in got:
+        y = y.cpu().numpy()
+        assert np.array_equal(bits(y)[ok], bits(want)[ok]) and np.isnan(y[~ok]).all()
