@@ -196,6 +196,8 @@ class ExpertParallelMoE(nn.Module):
         T, dev = x2d.shape[0], x2d.device
         mode, group_k, group_n = st["model"]
         xq = self._dispatch(x2d, st["src_rows"], None, None)
+        if xq.dtype != torch.float16:                                  # as the accumulation operators convert their operand
+            xq = xq.half()
         n, E = xq.shape[0], self.num_experts
         a, b = (torch.empty((n, self.inter), dtype=torch.float16, device=dev) for _ in range(2))
         gemm_grouped(xq, st["offsets"], [ex.w1.weight for ex in self.experts] + [ex.w3.weight for ex in self.experts],

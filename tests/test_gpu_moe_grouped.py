@@ -56,6 +56,23 @@ def test_grouped_experts_equal_one_at_a_time(ops, E, top_k, tokens):
     assert H.gemm_status() == 0
 
 
+@pytest.mark.parametrize("ops", ["fp16", "fp16_quant"])
+@pytest.mark.parametrize("packed", [False, True])
+def test_block_quantizer_that_yields_bf16(ops, packed):
+    """The accumulation operators convert their operand to fp16, so the grouped products see the same values."""
+    moe = _block(4, 2, 256, 640, _ops(ops))
+    moe.aq.out_dtype = torch.bfloat16
+    moe.packed_dispatch = packed
+    x = torch.randn((50, 256), device="cuda").half()
+    with torch.inference_mode():
+        assert moe._grouped_model() is not None
+        got = moe(x)
+        moe.experts[0].register_forward_hook(lambda m, i, o: None)
+        want = moe(x)
+    assert got.dtype == want.dtype == torch.float16
+    assert torch.equal(got.view(torch.int16), want.view(torch.int16))
+
+
 def test_expert_ids_of_another_integer_type():
     """A block with a router of its own that returns 32-bit ids: the same result as with 64-bit ones."""
     import hbq_b200 as H
