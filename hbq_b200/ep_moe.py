@@ -152,7 +152,7 @@ class ExpertParallelMoE(nn.Module):
             return None
         ex0 = self.experts[0]
         model = _accumulation(ex0.w1.ops)
-        if model is None or not isinstance(ex0.w2.aq, _CudaBlockQuantizer) or getattr(ex0.w2.aq, "keep_l2_scale", False):
+        if model is None or not isinstance(ex0.w2.aq, _CudaBlockQuantizer):
             return None
         fmt = ex0.w2.aq._format()
         key = [getattr(fmt, n) for n, _ in fmt._fields_]
@@ -163,7 +163,7 @@ class ExpertParallelMoE(nn.Module):
             return None
         for ex in self.experts:
             if type(ex) is not QuantExpert or _hooked(ex) or type(ex.w2.aq) is not type(ex0.w2.aq) or ex.w2.aq.out_dtype is not None or \
-                    _hooked(ex.w2.aq):
+                    getattr(ex.w2.aq, "keep_l2_scale", False) or _hooked(ex.w2.aq):
                 return None
             f = ex.w2.aq._format()
             if [getattr(f, n) for n, _ in f._fields_] != key:

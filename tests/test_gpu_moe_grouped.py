@@ -73,6 +73,22 @@ def test_block_quantizer_that_yields_bf16(ops, packed):
     assert torch.equal(got.view(torch.int16), want.view(torch.int16))
 
 
+@pytest.mark.parametrize("which", [0, 2])
+def test_an_expert_that_keeps_its_scales(which):
+    """Any expert whose quantizer keeps the chosen scales has them after the call: the block runs expert by expert."""
+    import hbq_b200 as H
+    moe = _block(4, 2, 256, 640, _ops("fp16"))
+    x = torch.randn((50, 256), device="cuda").half()
+    with torch.inference_mode():
+        want = moe(x)
+        moe.experts[which].w2.aq = H.HBQQuantizer(keep_l2_scale=True, **ACT)
+        assert moe._grouped_model() is None
+        got = moe(x)
+    assert torch.equal(got.view(torch.int16), want.view(torch.int16))
+    rows = int((moe.route(x)[1] == which).sum())
+    assert moe.experts[which].w2.aq.shared_scale.shape == (rows, 640 // 128)
+
+
 def test_expert_ids_of_another_integer_type():
     """A block with a router of its own that returns 32-bit ids: the same result as with 64-bit ones."""
     import hbq_b200 as H
