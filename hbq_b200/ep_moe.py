@@ -33,7 +33,7 @@ from .gemm import gemm_grouped
 from .kvcache import swiglu_quantize
 from .module import QLinear
 from .ops import FP16AccumMatMul, FP32AccumMatMul
-from .quantizer import PackedTensor, _CudaBlockQuantizer, _ptr, _QBase, _stream_ptr, dequantize_packed
+from .quantizer import PackedTensor, _CudaBlockQuantizer, _ptr, _QBase, _stream_ptr, dequantize_packed, hooked
 
 
 def _world(group) -> int:
@@ -44,15 +44,11 @@ def _rank(group) -> int:
     return dist.get_rank(group) if dist.is_available() and dist.is_initialized() else 0
 
 
-def _hooked(m: nn.Module) -> bool:
-    return bool(m._forward_hooks or m._forward_pre_hooks or "forward" in m.__dict__ or nn.modules.module._has_any_global_hook())
-
-
 def _accumulation(ops):
     """``(mode, group_k, group_n)`` of a linear layer's accumulation operator where the grouped GEMM has that model."""
-    if type(ops) is FP32AccumMatMul and not _hooked(ops):
+    if type(ops) is FP32AccumMatMul and not hooked(ops):
         return _lib.ACC_FP32, 0, 0
-    if type(ops) is FP16AccumMatMul and not _hooked(ops) and ops.group_size in (64, 128):
+    if type(ops) is FP16AccumMatMul and not hooked(ops) and ops.group_size in (64, 128):
         if ops.quant_block_size is None:
             return _lib.ACC_GROUPED, ops.group_size, 0
         if ops.quant_block_size == 32:
@@ -162,20 +158,20 @@ class ExpertParallelMoE(nn.Module):
         if dev.type != "cuda" or self.hidden % 8 or self.inter % 8:
             return None
         for ex in self.experts:
-            if type(ex) is not QuantExpert or _hooked(ex) or type(ex.w2.aq) is not type(ex0.w2.aq) or ex.w2.aq.out_dtype is not None or \
-                    getattr(ex.w2.aq, "keep_l2_scale", False) or _hooked(ex.w2.aq):
+            if type(ex) is not QuantExpert or hooked(ex) or type(ex.w2.aq) is not type(ex0.w2.aq) or ex.w2.aq.out_dtype is not None or \
+                    getattr(ex.w2.aq, "keep_l2_scale", False) or hooked(ex.w2.aq):
                 return None
             f = ex.w2.aq._format()
             if [getattr(f, n) for n, _ in f._fields_] != key:
                 return None
             for lin, shape in ((ex.w1, (self.inter, self.hidden)), (ex.w3, (self.inter, self.hidden)), (ex.w2, (self.hidden, self.inter))):
                 w = lin.weight
-                if (type(lin) is not QLinear or _hooked(lin) or lin.bias is not None or lin.check_finite or lin.w4_weight is not None
-                        or type(lin.yq) is not _QBase or _hooked(lin.yq) or _accumulation(lin.ops) != model
+                if (type(lin) is not QLinear or hooked(lin) or lin.bias is not None or lin.check_finite or lin.w4_weight is not None
+                        or type(lin.yq) is not _QBase or hooked(lin.yq) or _accumulation(lin.ops) != model
                         or w.dtype != torch.float16 or w.device != dev or tuple(w.shape) != shape or not w.is_contiguous()
                         or w.data_ptr() % 16):
                     return None
-                if lin is not ex.w2 and (type(lin.aq) is not _QBase or _hooked(lin.aq)):
+                if lin is not ex.w2 and (type(lin.aq) is not _QBase or hooked(lin.aq)):
                     return None
         return model
 

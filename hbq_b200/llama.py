@@ -38,7 +38,7 @@ from .fused import rmsnorm_quantize, softmax_quantize
 from .ep_moe import ExpertParallelMoE
 from .module import QLinear
 from .ops import FP16AccumMatMul, FP32AccumMatMul
-from .quantizer import _CudaBlockQuantizer, _QBase
+from .quantizer import _CudaBlockQuantizer, _QBase, calls_only_its_format
 
 
 @dataclass
@@ -71,10 +71,6 @@ def rope_tables(T: int, head_dim: int, theta: float, device, offset: int = 0):
     freqs = torch.outer(pos, inv)
     emb = torch.cat((freqs, freqs), dim=-1)
     return emb.cos().to(torch.float16)[None], emb.sin().to(torch.float16)[None]
-
-
-def _hooked(m: nn.Module) -> bool:
-    return bool(m._forward_hooks or m._forward_pre_hooks or "forward" in m.__dict__ or "q" in m.__dict__)
 
 
 def _same_format(a, b) -> bool:
@@ -144,7 +140,7 @@ class QLlamaAttention(nn.Module):
         c = self.query_chunk
         in_runs = q_len > c and q_len % c == 0 and c % 128 == 0
         Q = Qr = None
-        if in_runs and self.quant_post_rope_q and not _hooked(self.q_proj.aq):
+        if in_runs and self.quant_post_rope_q and calls_only_its_format(self.q_proj.aq):
             Qr = kvcache.quantize_q_runs(q, H, G, c, self.q_proj.aq, cos, sin)
         if Qr is not None:
             pass
@@ -180,7 +176,7 @@ class QLlamaAttention(nn.Module):
             Q5 = Q.contiguous().view(bsz, Hkv, G, q_len, D) if Qr is None else None
             O4 = torch.empty((bsz, q_len, H, D), dtype=q.dtype, device=q.device)
             # o_proj's input quantizer, where its blocks are heads, runs on each run's output while it is put in place
-            oq = self.o_proj.aq if not _hooked(self.o_proj.aq) else None
+            oq = self.o_proj.aq if calls_only_its_format(self.o_proj.aq) else None
             for t0 in range(0, q_len, c):
                 t1 = t0 + c
                 Qc = Q5[:, :, :, t0:t1].reshape(bsz, Hkv, G * c, D) if Qr is None else Qr[t0 // c]

@@ -145,6 +145,20 @@ class _QBase(nn.Module):
         return self.q(x)
 
 
+def hooked(m: nn.Module) -> bool:
+    """A call of ``m`` runs more than its class's ``forward``: hooks of its own or of every module, or a method put on
+    the object."""
+    return bool(m._forward_hooks or m._forward_pre_hooks or "forward" in m.__dict__ or "q" in m.__dict__
+                or nn.modules.module._has_any_global_hook())
+
+
+def calls_only_its_format(q) -> bool:
+    """``q(x)`` is the kernel of ``q``'s format and nothing else, so that a kernel which fuses that format may stand in
+    for the call: a block quantizer without hooks whose class keeps the library's ``forward`` and ``q``."""
+    return (isinstance(q, _CudaBlockQuantizer) and not hooked(q) and type(q).forward is _QBase.forward
+            and type(q).q in (_CudaBlockQuantizer.q, HBQQuantizer.q))
+
+
 class _CudaBlockQuantizer(_QBase):
     """Shared launch logic of the three block quantizers.
 

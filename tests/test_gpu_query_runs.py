@@ -59,3 +59,55 @@ def test_formats_that_are_refused():
         assert not kvcache.quantize_head_rows(x, out, 0, q)
         assert kvcache.quantize_q_runs(x.view(1, 16, 256), 2, 1, 8, q, cos, cos) is None
     assert not out.any()
+
+
+def _attention(o_aq):
+    import hbq_b200 as H
+    torch.manual_seed(1)
+    at = H.QLlamaAttention(H.LlamaArch(hidden=256, heads=2, kv_heads=1, head_dim=128, ffn=256, vocab=64, layers=1), device="cuda")
+    for lin in (at.q_proj, at.k_proj, at.v_proj, at.o_proj):
+        lin.weight.data.normal_(0, 0.05)
+        lin.aq = _quantizer(128, 2, 8)
+    at.quant_post_rope_q = True
+    at.o_proj.aq = o_aq
+    at.query_chunk = 128
+    return at
+
+
+@pytest.mark.parametrize("how", ["method", "forward", "hook", "global hook"])
+@pytest.mark.parametrize("T", [128, 256])
+def test_output_quantizers_that_do_more_than_their_format(how, T):
+    """A quantizer type with a `q` or `forward` of its own, or with hooks, is called at every length, also where the
+    attention runs in pieces (two at 256 tokens) whose output its format's kernel could quantise in place."""
+    import hbq_b200 as H
+    calls = []
+
+    class Method(H.HBQQuantizer):
+        def q(self, x):
+            calls.append(1)
+            return super().q(x)
+
+    class Forward(H.HBQQuantizer):
+        def forward(self, x):
+            calls.append(1)
+            return super().forward(x)
+
+    kind = {"method": Method, "forward": Forward}.get(how, H.HBQQuantizer)
+    oq = kind(128, 2, 2, 5, 3, l2_block_size=8, l2_sc_bit=2, l2_scheme="SIG-1")
+    handle = None
+    if how == "hook":
+        handle = oq.register_forward_hook(lambda m, i, o: calls.append(1))
+    if how == "global hook":
+        handle = torch.nn.modules.module.register_module_forward_hook(lambda m, i, o: calls.append(1) if m is oq else None)
+    x = torch.randn((T, 256), device="cuda").half()
+    cos = torch.ones((1, T, 128), device="cuda").half()
+    try:
+        with torch.no_grad():
+            got = _attention(oq)(x, 1, T, cos, torch.zeros_like(cos))
+    finally:
+        if handle is not None:
+            handle.remove()
+    assert len(calls) == 1
+    with torch.no_grad():
+        want = _attention(_quantizer(128, 2, 8))(x, 1, T, cos, torch.zeros_like(cos))
+    assert _same(got, want)
