@@ -35,11 +35,12 @@ def apply_rope(x: torch.Tensor, cos: torch.Tensor, sin: torch.Tensor) -> torch.T
 
 def rope_heads(x: torch.Tensor, num_heads: int, cos: torch.Tensor, sin: torch.Tensor) -> torch.Tensor:
     """``apply_rope(x.view(B, T, H, D).transpose(1, 2), cos, sin)`` for a projection output ``x [B, T, H * D]``, in one pass
-    where ``hbq_rope_heads`` takes it (fp16 CUDA tensors without a gradient to record), else the separate ops."""
+    where ``hbq_rope_heads`` takes it (fp16 CUDA tensors without a gradient to record, tables of every token for one or
+    all sequences), else the separate ops, which broadcast the tables."""
     B, T = x.shape[0], x.shape[1]
     D = _head_dim(x, num_heads)
     if x.is_cuda and x.dtype == torch.float16 and cos.dtype == torch.float16 and sin.dtype == torch.float16 and \
-            cos.device == x.device and sin.device == x.device and cos.dim() == 3 and \
+            cos.device == x.device and sin.device == x.device and cos.shape == sin.shape and tuple(cos.shape) in ((1, T, D), (B, T, D)) and \
             not (torch.is_grad_enabled() and (x.requires_grad or cos.requires_grad or sin.requires_grad)):
         xc = x.contiguous()
         c, s, rope_rows = _tables(cos, sin, B, T, D)

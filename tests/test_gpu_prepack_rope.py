@@ -51,3 +51,19 @@ def test_rope_without_a_quantizer(B, T, heads, D, per_batch):
         got = kvcache.rope_heads(x, heads, cos, sin)
     assert got.is_contiguous() and torch.equal(got.view(torch.int16), want.contiguous().view(torch.int16))
     assert kvcache.rope_heads(x.clone().requires_grad_(), heads, cos, sin).requires_grad
+
+
+@pytest.mark.parametrize("cos_shape,sin_shape", [((1, 1, 64), (1, 1, 64)), ((1, 9, 64), (3, 9, 64)), ((3, 9, 1), (3, 9, 1)), ((9, 64), (9, 64))])
+def test_rope_tables_that_broadcast(cos_shape, sin_shape):
+    from hbq_b200 import kvcache
+    x = torch.randn((3, 9, 2 * 64), device="cuda").half()
+    cos, sin = torch.rand(cos_shape, device="cuda").half(), torch.rand(sin_shape, device="cuda").half()
+    heads = x.view(3, 9, 2, 64).transpose(1, 2)
+    with torch.no_grad():
+        try:
+            want = kvcache.apply_rope(heads, cos, sin)
+        except RuntimeError:
+            with pytest.raises(RuntimeError):
+                kvcache.rope_heads(x, 2, cos, sin)
+            return
+        assert torch.equal(kvcache.rope_heads(x, 2, cos, sin), want)
