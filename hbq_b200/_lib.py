@@ -108,15 +108,34 @@ def lib() -> ctypes.CDLL:
 _host = None
 
 
+class _NoHost:
+    """Where torch has no CUDA the module cannot be built, and no call has a tensor for it: each takes the general path."""
+
+    @staticmethod
+    def quantize(*args):
+        return None
+
+    gemm = gemm_w4 = quantize
+
+    @staticmethod
+    def current_stream(index):
+        import torch
+        return torch.cuda.current_stream(index).cuda_stream
+
+
 def host():
     """The torch-facing module of the hot entry points (``csrc/host.cpp``), bound to this process's library."""
     global _host
     if _host is not None:
         return _host
+    from . import build            # (loads torch, whose libraries the module links against)
+    if build.host_tag() is None:
+        _host = _NoHost
+        return _host
     L = lib()
-    if not os.path.exists(HOST_PATH):
-        raise HbqError(f"{HOST_PATH} is missing: build it with `python -m hbq_b200.build`")
-    import torch  # noqa: F401  (the module links against torch's libraries, which this loads)
+    if not build.host_matches(HOST_PATH):
+        raise HbqError(f"{HOST_PATH} is missing or was built for another torch or Python than this process has "
+                       f"({build.host_tag()}): build it with `python -m hbq_b200.build`")
     loader = importlib.machinery.ExtensionFileLoader("hbq_host", HOST_PATH)
     m = importlib.util.module_from_spec(importlib.util.spec_from_loader("hbq_host", loader))
     loader.exec_module(m)

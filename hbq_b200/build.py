@@ -2,7 +2,8 @@
 torch-facing entry points (``csrc/host.cpp``) into ``lib/hbq_host.so``.
 
 The library targets sm_100a only and depends on nothing but the CUDA runtime, so it
-cross-compiles on a machine without a GPU; the module is built against the installed torch::
+cross-compiles on a machine without a GPU; the module is built against the installed torch (and is left out where that
+has no CUDA) and rebuilt when torch or Python has changed::
 
     python -m hbq_b200.build
 """
@@ -41,29 +42,55 @@ def is_stale() -> bool:
     return _older(LIB_PATH, [os.path.join(CSRC, s) for s in SOURCES] + HEADERS)
 
 
-def _host_command():
+def host_tag():
+    """What ``hbq_host.so`` is compiled for -- torch, its CUDA and C++ ABI, this Python; None where torch has no CUDA."""
+    import torch
+    if torch.version.cuda is None:
+        return None
+    return (f"hbq_host for torch {torch.__version__} cuda {torch.version.cuda} cxx11abi {int(torch._C._GLIBCXX_USE_CXX11_ABI)} "
+            f"python {sysconfig.get_config_var('SOABI')}")
+
+
+def host_matches(path=None) -> bool:
+    """The module at ``path`` (the built one) carries this process's tag."""
+    tag, path = host_tag(), path or HOST_PATH
+    if tag is None or not os.path.exists(path):
+        return False
+    with open(path, "rb") as f:
+        return tag.encode() + b"\0" in f.read()
+
+
+def host_is_stale() -> bool:
+    return host_tag() is not None and (_older(HOST_PATH, [HOST_SOURCE, HEADERS[-1]]) or not host_matches())
+
+
+def _host_command(out: str):
     import torch
     root = os.path.dirname(torch.__file__)
     cuda = os.path.dirname(os.path.dirname(_nvcc()))
     inc = [os.path.join(root, "include"), os.path.join(root, "include", "torch", "csrc", "api", "include"),
            sysconfig.get_paths()["include"], os.path.join(cuda, "include")]
-    return ["g++", "-O2", "-std=c++17", "-fPIC", "-shared", "-o", HOST_PATH, HOST_SOURCE, *["-I" + i for i in inc],
+    return ["g++", "-O2", "-std=c++17", "-fPIC", "-shared", f"-D_GLIBCXX_USE_CXX11_ABI={int(torch._C._GLIBCXX_USE_CXX11_ABI)}",
+            f'-DHBQ_HOST_TAG="{host_tag()}"', "-o", out, HOST_SOURCE, *["-I" + i for i in inc],
             "-L" + os.path.join(root, "lib"), "-lc10", "-lc10_cuda", "-ltorch_cpu", "-ltorch_cuda", "-ltorch", "-ltorch_python"]
 
 
 def build_library(force: bool = False, verbose: bool = False) -> str:
-    """Compile what is missing or older than its sources; return the library's path."""
+    """Compile what is missing or out of date; return the library's path."""
     host = None
     os.makedirs(LIB_DIR, exist_ok=True)
-    if force or _older(HOST_PATH, [HOST_SOURCE, HEADERS[-1]]):
+    made = f"{HOST_PATH}.{os.getpid()}"                                  # renamed when complete: the old one may be loaded
+    if host_tag() is not None and (force or host_is_stale()):
         env = {k: v for k, v in os.environ.items() if k not in ("CC", "CXX")}
-        host = subprocess.Popen(_host_command(), env=env)               # beside nvcc
+        host = subprocess.Popen(_host_command(made), env=env)           # beside nvcc
     try:
         if force or is_stale():
             _build_cuda(verbose)
     finally:
-        if host is not None and host.wait() != 0:
-            raise RuntimeError("building hbq_host.so failed")
+        if host is not None:
+            if host.wait() != 0:
+                raise RuntimeError("building hbq_host.so failed")
+            os.replace(made, HOST_PATH)
     return LIB_PATH
 
 

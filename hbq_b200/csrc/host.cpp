@@ -15,6 +15,9 @@
 
 namespace {
 
+// What this module was compiled for (build.py compares it with the process that is about to load it).
+__attribute__((used)) const char built_for[] = HBQ_HOST_TAG;
+
 decltype(&hbq_quantize) p_quantize = nullptr;
 decltype(&hbq_gemm) p_gemm = nullptr;
 decltype(&hbq_gemm_workspace_bytes) p_gemm_workspace_bytes = nullptr;
