@@ -28,7 +28,7 @@ EXPORTS = [
     "hbq_gemm_kn_noalloc", "hbq_gemm_w4", "hbq_gemm_w4_prepack", "hbq_gemm_w4_prepacked_bytes",
     "hbq_gemm_w4_workspace_bytes", "hbq_kv_write_k", "hbq_kv_write_v", "hbq_swiglu_quantize", "hbq_rmsnorm_quantize", "hbq_softmax_quantize",
     "hbq_rope_heads", "hbq_quantize_q_runs", "hbq_quantize_head_rows", "hbq_moe_route", "hbq_gemm_grouped", "hbq_moe_combine",
-    "hbq_gemm_status", "hbq_gemm_status_reset", "hbq_gemm_wait_selftest", "hbq_gemm_reserve_sms", "hbq_error_string", "hbq_last_cuda_error",
+    "hbq_gemm_status", "hbq_gemm_status_reset", "hbq_gemm_wait_selftest", "hbq_gemm_reserve_sms", "hbq_gemm_tile_columns", "hbq_error_string", "hbq_last_cuda_error",
     "hbq_version", "hbq_launch_count",
 ]
 
@@ -97,6 +97,7 @@ def lib() -> ctypes.CDLL:
     L.hbq_gemm_status.argtypes = [ctypes.POINTER(ci)]
     L.hbq_gemm_wait_selftest.argtypes = [vp, vp, vp, i64, i64, i64, ci, ci, ci, ctypes.c_uint32, vp]
     L.hbq_gemm_reserve_sms.argtypes = [ci]
+    L.hbq_gemm_tile_columns.argtypes = [i64, i64, ci, ci]
     L.hbq_error_string.argtypes = [ci]
     L.hbq_error_string.restype = ctypes.c_char_p
     L.hbq_last_cuda_error.restype = ctypes.c_char_p

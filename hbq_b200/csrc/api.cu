@@ -84,6 +84,8 @@ int transpose_launch(const void*, void*, int64_t, int64_t, cudaStream_t);
 int gemm_tc_status(int*);
 int gemm_tc_status_reset();
 int gemm_tc_reserve_sms(int n);
+int gemm_tc_usable_sms(int*);
+int gemm_tc_tile_width(int64_t, int64_t, int, int);
 int gemm_tc_grouped_launch(const void*, int64_t, const int*, int, const void* const*, void* const*, const int*, int64_t, int64_t, int,
                            int, int, cudaStream_t);
 int moe_route_launch(const int64_t*, int64_t, int, int, int*, int64_t*, int*, cudaStream_t);                      // moe.cu
@@ -353,6 +355,12 @@ int hbq_gemm_status(int* status_host)
 }
 int hbq_gemm_status_reset(void) { return gemm_tc_status_reset(); }
 int hbq_gemm_reserve_sms(int n) { return gemm_tc_reserve_sms(n); }
+int hbq_gemm_tile_columns(int64_t M, int64_t N, int mode, int sms)
+{
+    if (M <= 0 || N <= 0) return HBQ_ERR_ARG;
+    if (sms <= 0) { const int rc = gemm_tc_usable_sms(&sms); if (rc) return rc; }
+    return gemm_tc_tile_width((M + 127) / 128, N, sms, mode);
+}
 
 const char* hbq_error_string(int code)
 {

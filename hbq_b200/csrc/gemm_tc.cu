@@ -132,7 +132,7 @@ struct TcArgs {
     int k_stages;        // ceil(K / 64)
     int chunk_k16;       // MMAs (K = 16 each) per accumulation chunk
     int issuers;         // MMA-issuing warps to use (1 or 2)
-    int bn;              // tile width chosen by the host: 256, or 128 for decode-sized M
+    int bn;              // tile width chosen by the host (gemm_tc_tile_width): 256, 192 or 128
     uint32_t poll_limit; // polls after which a wait on an mbarrier gives up (kDefaultPollLimit)
     int withhold_loads;  // self-test of the give-up path: the producer issues no load at all, so every
                          // consumer wait runs out with nothing in flight
@@ -552,13 +552,14 @@ bool gemm_tc_eligible(int64_t M, int64_t N, int64_t K, int mode, int group_k, in
     return true;
 }
 
-// Tile width: all CTAs of a round work on tiles of one width, so the time is (rounds) x (width).  256 columns as a rule: a
+// Tile width for a launch on `sms` SMs (those that hbq_gemm_reserve_sms keeps free do not count): all CTAs of a round
+// work on tiles of one width, so the time is (rounds) x (width).  256 columns as a rule: a
 // narrower tile reads A again for less work and a column of it costs some 15 % more (forced to 192: 4096 x 4096 x 4096
 // 105 -> 119 us; to 224: 4096 x 14336 x 4096 343 -> 360 us, though both save 5 % of rounds x width).  192 where they take
 // no more rounds (1000 x 6144 x 4096, 192 tiles of 256 or 256 of 192 in two rounds of 148: fp32 53.8 -> 48.0 us, grouped
 // fp16 sums 59.6 -> 50.5), for the accumulation models whose drain of an accumulator is shorter than its MMAs; 128 where
 // 256-column tiles would leave more than half of the SMs without work, or for N of at most 128.
-static int tile_width(int64_t tiles_m, int64_t N, int sms, int mode)
+int gemm_tc_tile_width(int64_t tiles_m, int64_t N, int sms, int mode)
 {
     const int64_t t256 = tiles_m * ((N + 255) / 256), t192 = tiles_m * ((N + 191) / 192);
     if (N <= 128 || t256 * 2 <= sms) return 128;
@@ -595,6 +596,15 @@ int transpose_launch(const void* in, void* out, int64_t R, int64_t Ccols, cudaSt
 // SMs that launches leave free for a kernel of another stream (hbq_gemm_reserve_sms)
 static std::atomic<int> g_reserved_sms{0};
 
+int gemm_tc_usable_sms(int* usable)
+{
+    int sms = 0;
+    { const int rc = device_sms(&sms); if (rc) return rc; }
+    const int n = sms - g_reserved_sms.load();
+    *usable = n > 0 ? n : 1;
+    return HBQ_OK;
+}
+
 // A [M,K], W [N,K], both fp16 row-major and 16-byte aligned.
 // poll_limit = 0: the default bound; withhold_loads: see TcArgs (the self-test of hbq_gemm_wait_selftest).
 int gemm_tc_launch_ex(const void* A, const void* W, void* C, int64_t M, int64_t N, int64_t K, int mode,
@@ -612,10 +622,10 @@ int gemm_tc_launch_ex(const void* A, const void* W, void* C, int64_t M, int64_t 
     TcArgs args;
     args.C = (__half*)C; args.bias = (const __half*)bias;
     args.M = (int)M; args.N = (int)N; args.K = (int)K;
-    int sms = 0;
-    { const int rc2 = device_sms(&sms); if (rc2) return rc2; }
+    int usable = 0;
+    { const int rc2 = gemm_tc_usable_sms(&usable); if (rc2) return rc2; }
     args.tiles_m = (int)((M + BM - 1) / BM);
-    args.bn = tile_width(args.tiles_m, N, sms, mode);
+    args.bn = gemm_tc_tile_width(args.tiles_m, N, usable, mode);
     args.tiles_n = (int)((N + args.bn - 1) / args.bn);
     rc = make_map(&mb, W, N, K, args.bn);
     if (rc) return rc;
@@ -626,7 +636,6 @@ int gemm_tc_launch_ex(const void* A, const void* W, void* C, int64_t M, int64_t 
     args.withhold_loads = withhold_loads;
 
     const int64_t total = (int64_t)args.tiles_m * args.tiles_n;
-    const int usable = sms - g_reserved_sms.load() > 0 ? sms - g_reserved_sms.load() : 1;
     const int grid = (int)(total < usable ? total : usable);
 
     switch (mode) {
@@ -684,8 +693,8 @@ int gemm_tc_grouped_launch(const void* A, int64_t rows, const int* offsets, int 
     uintptr_t bits = reinterpret_cast<uintptr_t>(A);
     for (int i = 0; i < entries; ++i) bits |= reinterpret_cast<uintptr_t>(W[i]) | reinterpret_cast<uintptr_t>(C[i]);
     if (bits & 15) return HBQ_ERR_ALIGN;
-    int sms = 0;
-    { const int rc = device_sms(&sms); if (rc) return rc; }
+    int usable = 0;
+    { const int rc = gemm_tc_usable_sms(&usable); if (rc) return rc; }
     CUtensorMap ma;
     { const int rc = make_map(&ma, A, rows, K, BM); if (rc) return rc; }
     TcArgs args;
@@ -697,13 +706,12 @@ int gemm_tc_grouped_launch(const void* A, int64_t rows, const int* offsets, int 
     for (int i = 0; i < entries; ++i) experts = experts > expert[i] + 1 ? experts : expert[i] + 1;
     const int64_t rows_tiles = rows < experts ? rows : rows / BM + (experts + 1) / 2;
     const int64_t tiles_m = rows_tiles * n0 / experts > 0 ? rows_tiles * n0 / experts : 1;
-    args.bn = tile_width(tiles_m, N, sms, mode);
+    args.bn = gemm_tc_tile_width(tiles_m, N, usable, mode);
     args.tiles_n = (int)((N + args.bn - 1) / args.bn);
     args.k_stages = (int)((K + BK - 1) / BK);
     args.chunk_k16 = (mode == HBQ_ACC_FP32) ? args.k_stages * (BK / 16) : group_k / 16;
     args.issuers = 2;
     args.poll_limit = kDefaultPollLimit;
-    const int usable = sms - g_reserved_sms.load() > 0 ? sms - g_reserved_sms.load() : 1;
     for (int e0 = 0; e0 < entries; e0 += TC_MAX_ENTRIES) {
         GroupArgs g;
         memset(&g, 0, sizeof(g));

@@ -320,6 +320,10 @@ int hbq_gemm_w4(const void* X, const void* Wp, void* C, int64_t M, int64_t N, in
  * the previous value.  Host-side setting read at launch time; no reference counterpart. */
 int hbq_gemm_reserve_sms(int n);
 
+/* Columns of the output tiles (128, 192 or 256; 128 rows each) with which the tensor-core kernel computes an [M, N]
+ * result on `sms` SMs; sms <= 0: those of the current device that hbq_gemm_reserve_sms leaves. */
+int hbq_gemm_tile_columns(int64_t M, int64_t N, int mode, int sms);
+
 /* ---- misc ------------------------------------------------------------------------------ */
 
 const char* hbq_error_string(int code);

@@ -42,3 +42,24 @@ def test_grouped_products(mode, group_k, rows):
         if n:
             assert torch.equal(out[r0:r0 + n], gemm(a[r0:r0 + n].contiguous(), w, mode, group_k, b_is_nk=True, force_simt=True))
         r0 += n
+
+
+def test_width_follows_the_sms_that_are_left():
+    """1000 x 6144: 192 tiles of 256 columns or 256 of 192, two rounds either way on 128 SMs and more; on fewer the
+    narrower tiles take a third round."""
+    import hbq_b200 as H
+    from hbq_b200 import _lib
+    from hbq_b200.gemm import gemm
+    L = _lib.lib()
+    sms = torch.cuda.get_device_properties(0).multi_processor_count
+    a = torch.randint(-4, 5, (1000, 320), device="cuda").half()
+    w = torch.randint(-3, 4, (6144, 320), device="cuda").half()
+    want = gemm(a, w, 0, b_is_nk=True)
+    prev = H.gemm_reserve_sms(0)
+    try:
+        for left, columns in ((148, 192), (128, 192), (127, 256), (100, 256), (96, 256)):
+            H.gemm_reserve_sms(sms - left)
+            assert L.hbq_gemm_tile_columns(1000, 6144, 0, 0) == columns == L.hbq_gemm_tile_columns(1000, 6144, 0, left)
+            assert torch.equal(gemm(a, w, 0, b_is_nk=True), want)
+    finally:
+        H.gemm_reserve_sms(prev)
