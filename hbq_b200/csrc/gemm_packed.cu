@@ -106,6 +106,18 @@ struct PkArgs {
     int split;                  // S >= 2: a tile's K range is split over the S CTAs of a cluster; 0: no clusters
 };
 
+// What the packed-weight kernels bring into L2 while the kernel before them still runs.  The tcgen05 kernel and the
+// one-token kernel ask only for what they read first: a CTA's whole run, queued ahead of that, costs more than it hides
+// wherever a kernel that ends at once or another product precedes.  us per call in a graph, separate weights, 16 tokens x
+// [14336, 4096], whole run / first records / nothing: behind a workspace fill 23.9 / 22.1 / 22.3, behind another product
+// 19.6 / 19.0 / 18.9, behind the tokens' quantizer 22.8 / 21.3 / 21.1 (33 tokens x [4096, 14336]: 25.6 / 24.2 / 24.6;
+// 16 x [4096, 4096]: 12.8 / 12.7 / 12.8).  One token x [14336, 4096]: 14.2 / 13.6 / 13.9 behind a product, 16.6 / 16.0 /
+// 16.2 behind the quantizer.  The warp-level-MMA kernel gains from its whole share: 8 tokens
+// 16.9 whole, 17.0 four blocks a warp, 17.5 nothing behind a product; 19.6 / 19.4 / 20.0 behind the quantizer; 19.0 / 19.5 /
+// 20.1 with weights that L2 still holds.
+constexpr int PK_PREFETCH = 4;                                // records of a CTA's run, in processing order (3 to 8: the same)
+constexpr int GV_PREFETCH = 2;                                // blocks of 128 k per warp (four: 13.7 and 16.2)
+
 __device__ __forceinline__ void l2_prefetch(const void* p) { asm volatile("prefetch.global.L2 [%0];" ::"l"(p)); }
 
 __device__ __forceinline__ uint32_t prmt(uint32_t a, uint32_t b, uint32_t sel)
@@ -309,12 +321,10 @@ gemm_packed_kernel(const __grid_constant__ CUtensorMap mapX, const __grid_consta
                      ::"r"(smem_u32(tmem_base_smem)), "r"(a.tmem_cols) : "memory");
         asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
     }
-    // the packed records of this CTA's run (one stretch of memory) on their way into L2 while the kernel before this one
-    // still runs
-    if (CB != 16 && warp == 6)
-        for (int i = lane; i < nst; i += 32)
-            asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;"
-                         ::"l"(a.wp + (int64_t)(g0 + i) * pk_rec_bytes(CB)), "r"(pk_rec_bytes(CB)) : "memory");
+    // the records that the pipeline asks for first on their way into L2 while the kernel before this one still runs
+    if (CB != 16 && warp == 6 && lane < min(nst, PK_PREFETCH))
+        asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;"
+                     ::"l"(a.wp + (int64_t)stage_g(lane) * pk_rec_bytes(CB)), "r"(pk_rec_bytes(CB)) : "memory");
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
@@ -803,9 +813,9 @@ __global__ void __launch_bounds__(512) gemv_packed_kernel(const GvArgs a)
     uint4* xs = reinterpret_cast<uint4*>(gv_smem);                               // [MT][K] fp16
     float* red = reinterpret_cast<float*>(gv_smem + (size_t)MT * a.K * 2);        // [ks][MT][32]
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    // while the kernel before this one (the tokens' quantizer) still runs: this CTA's weight on its way into L2 -- 32
-    // rows of every record, four runs of 512 bytes of codes and one of 256 of side words
-    for (int k = warp; k < a.nblk; k += a.ks) {
+    // while the kernel before this one (the tokens' quantizer) still runs: the first blocks of every warp on their way into
+    // L2 -- 32 rows of a record, four runs of 512 bytes of codes and one of 256 of side words
+    for (int k = warp; k < min(a.nblk, GV_PREFETCH * a.ks); k += a.ks) {
         const uint8_t* rec = a.wp + ((int64_t)(blockIdx.x >> 2) * a.nblk + k) * pk_rec_bytes(4);
         const int r0 = (blockIdx.x & 3) * 32;
         if (lane < 16) l2_prefetch(rec + ((lane >> 2) * PK_ROWS + r0) * 16 + (lane & 3) * 128);
@@ -921,7 +931,7 @@ __global__ void __launch_bounds__(512) gemm_packed_reg_kernel(const RgArgs a)
     const int slab = warp % a.slabs, ksp = warp / a.slabs;
     const int row0 = (blockIdx.x * a.slabs + slab) * 32, tile = row0 >> 7, rt = row0 & (PK_ROWS - 1);
     const uint8_t* rec0 = a.wp + (int64_t)tile * a.nblk * pk_rec_bytes(4);
-    for (int k = ksp; k < a.nblk; k += a.ks) {                                  // as in gemv_packed_kernel
+    for (int k = ksp; k < a.nblk; k += a.ks) {                                  // as in gemv_packed_kernel, the warp's whole share
         const uint8_t* rec = rec0 + (int64_t)k * pk_rec_bytes(4);
         if (lane < 16) l2_prefetch(rec + ((lane >> 2) * PK_ROWS + rt) * 16 + (lane & 3) * 128);
         else if (lane < 18) l2_prefetch(rec + pk_code_bytes(4) + rt * 8 + (lane & 1) * 128);
