@@ -183,3 +183,16 @@ def test_cuda_graph_capture_of_a_decode_step():
             torch.cuda.synchronize()
             assert torch.equal(y_static, lin(x_new))
     assert H.gemm_status() == 0
+
+
+@pytest.mark.parametrize("rows,N,K", [(1, 256, 512), (1, 128, 49280), (2, 1024, 4096), (5, 256, 640), (8, 19200, 256)])
+def test_up_to_eight_rows_leave_the_workspace_alone(rows, N, K):
+    """The workspace of these calls is not zeroed: whatever it holds, it neither changes the result nor is changed."""
+    w4, deq = _weight("hbq_a_wgt", N, K, rows + N)
+    x = torch.randn((rows, K), device="cuda").half()
+    ref = x.double() @ deq.double().t()
+    for fill in (0xFF, 0x00, 0x5A):
+        w4._workspace(rows).fill_(fill)
+        y = w4.matmul(x)
+        assert float((y.double() - ref).norm() / ref.norm()) <= REL_TOL
+        assert bool((w4._workspace(rows) == fill).all())
