@@ -610,7 +610,9 @@ __global__ void __launch_bounds__(TAB_THREADS, 2) hbq_tab_kernel(const TabArgs a
 // everything else once.  The totals are added in the order of the tree over the block's chunks that the other kernels
 // use (chunk distance 8, 4, 2, 1), so a sum that the fp32 additions round is the same number in all of them.
 // Bound: instruction issue (about twice hbq_tab_kernel's work per element).  Weight [14336, 4096] to packed planes:
-// 136 us; the arithmetic kernel of quantize.cu, which alone had these outputs, took 507 us.
+// 139 us; the arithmetic kernel of quantize.cu, which alone had these outputs, took 507 us.  The tensor alone: 118 us with
+// micro-blocks of 8, 130 with 32 (NaNs put over the stored values; patched before the store: 122 and 127; infinities and
+// NaNs read as zeros: 114 and 128).
 // An infinite |x|, whose quotient comes out of the division as NaN, takes the largest level: the minimum, which drops
 // the NaN, is the inner one.
 template <int MB, int C, int ML, bool SMALL>
@@ -714,7 +716,15 @@ __global__ void __launch_bounds__(MIX_THREADS, 2) hbq_tab_mix_kernel(const TabAr
         for (int off = Gt >> 1; off >= 1; off >>= 1)
             mx = h2_bits(__hmax2_nan(bits_h2(mx), bits_h2(__shfl_xor_sync(0xFFFFFFFFu, mx, off))));
         const bool nans = max(mx & 0x7FFFu, (mx >> 16) & 0x7FFFu) > 0x7C00u;
+        uint32_t nan_elems = 0u;                                 // tensor alone: element j of chunk k at bit 8 k + j
         if (__any_sync(0xFFFFFFFFu, nans)) {
+            if (!SIDE) {
+                #pragma unroll
+                for (int k = 0; k < C; ++k)
+                    #pragma unroll
+                    for (int p = 0; p < 4; ++p)
+                        nan_elems |= (((xb[k][p] & 0x7FFFu) > 0x7C00u ? 1u : 0u) | (((xb[k][p] >> 16) & 0x7FFFu) > 0x7C00u ? 2u : 0u)) << (8 * k + 2 * p);
+            }
             mx = 0u;
             #pragma unroll
             for (int k = 0; k < C; ++k)
@@ -778,7 +788,7 @@ __global__ void __launch_bounds__(MIX_THREADS, 2) hbq_tab_mix_kernel(const TabAr
                 const __half2 dneg = small ? __hmul2(bits_h2(cw[p]), tlb) : __hmul2(__hmul2(bits_h2(cw[p]), bits_h2(nt)), bits_h2(l1u));
                 dq[p] = (h2_bits(dneg) & 0x7FFF7FFFu) | sg[p];
             }
-            if (nans) {                                 // a NaN stays one in the tensor; its code has all bits set (E2M2: no sign)
+            if (SIDE && nans) {                                  // a NaN stays one in the tensor; its code has all bits set (E2M2: no sign)
                 #pragma unroll
                 for (int p = 0; p < 4; ++p)
                     #pragma unroll
@@ -814,6 +824,11 @@ __global__ void __launch_bounds__(MIX_THREADS, 2) hbq_tab_mix_kernel(const TabAr
             }
         }
         if (SIDE) store_block_side(a, bi, Gt, valid && g == 0, l1b, second ? 1u : 0u, l2word);
+        else if (nan_elems != 0u && valid)                       // NaNs over what the chunks stored for them
+            for (uint32_t m = nan_elems; m != 0u; m &= m - 1u) {
+                const int i = __ffs(m) - 1;
+                reinterpret_cast<uint16_t*>(a.deq + c0 + (i >> 3) * Gt)[i & 7] = 0x7FFFu;
+            }
     }
 }
 
