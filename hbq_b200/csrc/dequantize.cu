@@ -1,6 +1,7 @@
 // Packed codes and scales -> fake-quantised fp16 / bf16 tensor (hbq_dequantize).
 //
-// Bound: HBM (codes and scales in, 2 bytes per element out).  A thread owns DQ_UNROLL chunks of 8 elements, one
+// Bound: issue slots (67 % used) and the half-rate ALU pipe (63 %): two bit fields and a candidate select per pair (codes
+// and scales in, 2 bytes per element out would take HBM 23 us).  A thread owns DQ_UNROLL chunks of 8 elements, one
 // CTA-width apart, so that its code words and scales are all in flight before the first is used and every warp
 // access is contiguous.  All planes are rows of whole blocks, so a chunk's block is its flat index shifted; only
 // the output address of a tensor with a padded last block needs the row.
@@ -10,7 +11,7 @@
 // exact multiply by 2^(15 - bias) decodes any format of up to five exponent bits; integers go through the pattern
 // of 1024 + v.  With five exponent bits the top field stands for 2^16 and more, beyond fp16: infinity whatever the
 // mantissa says, so the mantissa is cleared there (its pattern would be a NaN's).
-// HBQ weight [14336, 4096] (150 MB moved): 37 us = 4.0 TB/s; one chunk per thread with scalar ldexpf decoding and a
+// HBQ weight [14336, 4096] (150 MB moved): 37-39 us = 4.0 TB/s; one chunk per thread with scalar ldexpf decoding and a
 // 64-bit division each took 301 us.
 #include "quantize_dev.cuh"
 #include <string.h>

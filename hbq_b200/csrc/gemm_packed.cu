@@ -1401,7 +1401,7 @@ int gemm_w4_launch(const void* X, const void* Wp, void* C, int64_t M, int64_t N,
     { const int rc = device_sms(&sms); if (rc) return rc; }
     a.poll_limit = poll_limit ? poll_limit : (1u << 23);
     // the nibble container has two more kernels for the smallest batches (measured on B200, 16 / 8 / 1 tokens x
-    // [14336, 4096]: tcgen05 path 20.3 us, warp-level MMA 17.7 us, no tensor core 14.3 us).  Neither touches the
+    // [14336, 4096]: tcgen05 path 19.0 us, warp-level MMA 16.5 us, no tensor core 13.6 us).  Neither touches the
     // workspace: packed_gemm.py does not zero it for them.
     if (M == 1 && container_bits == 4 && K * 2 <= 96 * 1024)
         return w4_launch_gemv(X, Wp, C, M, N, K, a, ms, bias, sms, stream);

@@ -17,7 +17,9 @@
 //   * a thread owns C chunks (8 elements each) of ONE block, chunk g + k*Gt for lane g of the block's Gt
 //     lanes: the block maximum, the E5M3 scale and the division constants are computed once per C chunks,
 //     and every warp load / store still covers whole 32-byte sectors.
-// Results are bit-identical to the reference's eager fp16 quantizer (golden vectors + oracle tests).
+// Results are bit-identical to the reference's eager fp16 quantizer (golden vectors + oracle tests) for finite inputs.  An
+// infinite or NaN quotient takes the smallest level in the one-table kernels (their clamp's maximum, which drops a NaN, is
+// the inner one), so such an input becomes a zero; hbq_tab_mix_kernel keeps both.
 #include "quantize_tab.cuh"
 #include "vcache_dev.cuh"
 #include <mutex>
