@@ -157,6 +157,8 @@ class ExpertParallelMoE(nn.Module):
         dev = ex0.w1.weight.device
         if dev.type != "cuda" or self.hidden % 8 or self.inter % 8:
             return None
+        if model[0] == _lib.ACC_PSUM_INT8 and (self.hidden % model[1] or self.inter % model[1] or self.hidden % model[2] or self.inter % model[2]):
+            return None                                                # sizes that the operator refuses, with its message
         for ex in self.experts:
             if type(ex) is not QuantExpert or hooked(ex) or type(ex.w2.aq) is not type(ex0.w2.aq) or ex.w2.aq.out_dtype is not None or \
                     getattr(ex.w2.aq, "keep_l2_scale", False) or hooked(ex.w2.aq):

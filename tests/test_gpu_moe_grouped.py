@@ -89,6 +89,20 @@ def test_an_expert_that_keeps_its_scales(which):
     assert moe.experts[which].w2.aq.shared_scale.shape == (rows, 640 // 128)
 
 
+@pytest.mark.parametrize("hidden,inter", [(264, 640), (256, 648), (320, 608), (256, 640)])
+def test_sizes_that_the_partial_sum_operator_refuses(hidden, inter):
+    """K in whole groups of 64 and N in whole blocks of 32, as the operator of an expert's own layers asks for."""
+    moe = _block(4, 2, hidden, inter, _ops("fp16_quant"))
+    x = torch.randn((50, hidden), device="cuda").half()
+    with torch.inference_mode():
+        if hidden % 64 == 0 and inter % 64 == 0:
+            assert moe._grouped_model() is not None and moe(x).shape == x.shape
+        else:
+            assert moe._grouped_model() is None
+            with pytest.raises(RuntimeError, match="divisible"):
+                moe(x)
+
+
 def test_expert_ids_of_another_integer_type():
     """A block with a router of its own that returns 32-bit ids: the same result as with 64-bit ones."""
     import hbq_b200 as H
