@@ -448,7 +448,8 @@ gemm_tc_grouped_kernel(const __grid_constant__ CUtensorMap mapA, const __grid_co
         const int* const offsets = behind_wait(group.offsets);
         int n = 0;
         for (int e = 0; e < group.entries; ++e) {
-            const int r0 = offsets[group.expert[e]], r1 = offsets[group.expert[e] + 1];
+            // whatever the device holds there: no row outside A and C
+            const int r0 = min(max(offsets[group.expert[e]], 0), args.M), r1 = max(min(offsets[group.expert[e] + 1], args.M), r0);
             s_first[e] = n;
             s_rows[2 * e] = r0;
             s_rows[2 * e + 1] = r1;

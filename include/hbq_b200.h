@@ -259,7 +259,8 @@ int hbq_gemm_wait_selftest(const void* A, const void* W, void* C, int64_t M, int
  *                    A copy whose id is outside [0, experts) belongs to no expert: it is sorted behind offsets[experts]
  *                    and its pos is -1.
  *   hbq_gemm_grouped entry i: C_host[i][r, :] = A[r, :] * W_host[i][N, K]^T for the rows of expert expert_host[i], i.e.
- *                    offsets[e] .. offsets[e + 1] - 1; A [rows, K], accumulation model as hbq_gemm (FP32, GROUPED,
+ *                    offsets[e] .. offsets[e + 1] - 1, as far as they lie in [0, rows); A and C_host[i] have `rows` rows,
+ *                    offsets at least max(expert_host) + 2 entries; accumulation model as hbq_gemm (FP32, GROUPED,
  *                    PSUM_INT8 with group_n = 32).  W_host / C_host / expert_host are host arrays of `entries`.
  *   hbq_moe_combine  out[t, :] = sum_j fp16(y_rows[pos[t * top_k + j], :] * weights[t, j]) over the copies with pos >= 0. */
 int hbq_moe_route(const int64_t* ids, int64_t tokens, int top_k, int experts, int32_t* offsets, int64_t* src_rows,

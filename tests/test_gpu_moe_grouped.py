@@ -176,3 +176,24 @@ def test_ids_without_an_expert_are_left_out(E, tokens, top_k):
     for j in range(top_k):                               # the kernel's order: fp32 sums of the fp16 products
         want += parts[:, j]
     assert torch.equal(out, want.half())
+
+
+@pytest.mark.parametrize("offsets", [[0, 200, 1000], [-7, 130, 300], [0, 299, 301], [250, 100, 300], [400, 500, 600], [-9, -5, -1]])
+def test_row_offsets_outside_the_rows(offsets):
+    """Entries only compute and store the rows that A and C have; what lies around C stays as it was."""
+    from hbq_b200 import _lib
+    from hbq_b200.gemm import gemm, gemm_grouped
+    rows, K, N = 300, 128, 256
+    g = torch.Generator(device="cuda").manual_seed(5)
+    a = torch.randint(-4, 5, (rows, K), device="cuda", generator=g).half()
+    ws = [torch.randint(-3, 4, (N, K), device="cuda", generator=g).half() for _ in range(2)]
+    around = torch.full((rows + 2048, N), 7.0, dtype=torch.float16, device="cuda")
+    out = around[1024:1024 + rows]
+    gemm_grouped(a, torch.tensor(offsets, dtype=torch.int32, device="cuda"), ws, [out, out], range(2), _lib.ACC_FP32)
+    want = torch.full_like(around, 7.0)
+    for e in range(2):
+        r0 = min(max(offsets[e], 0), rows)
+        r1 = max(min(offsets[e + 1], rows), r0)
+        if r1 > r0:
+            want[1024 + r0:1024 + r1] = gemm(a[r0:r1].contiguous(), ws[e], 0, b_is_nk=True, force_simt=True)
+    assert torch.equal(around, want)
