@@ -39,7 +39,7 @@ def rope_heads(x: torch.Tensor, num_heads: int, cos: torch.Tensor, sin: torch.Te
     all sequences), else the separate ops, which broadcast the tables."""
     B, T = x.shape[0], x.shape[1]
     D = _head_dim(x, num_heads)
-    if x.is_cuda and x.dtype == torch.float16 and cos.dtype == torch.float16 and sin.dtype == torch.float16 and \
+    if x.is_cuda and x.numel() and x.dtype == torch.float16 and cos.dtype == torch.float16 and sin.dtype == torch.float16 and \
             cos.device == x.device and sin.device == x.device and cos.shape == sin.shape and tuple(cos.shape) in ((1, T, D), (B, T, D)) and \
             not (torch.is_grad_enabled() and (x.requires_grad or cos.requires_grad or sin.requires_grad)):
         xc = x.contiguous()

@@ -67,3 +67,11 @@ def test_rope_tables_that_broadcast(cos_shape, sin_shape):
                 kvcache.rope_heads(x, 2, cos, sin)
             return
         assert torch.equal(kvcache.rope_heads(x, 2, cos, sin), want)
+
+
+@pytest.mark.parametrize("B,T", [(0, 5), (2, 0)])
+def test_rope_of_nothing(B, T):
+    from hbq_b200 import kvcache
+    x, cos = torch.empty((B, T, 2 * 64), device="cuda").half(), torch.ones((1, T, 64), device="cuda").half()
+    with torch.no_grad():
+        assert kvcache.rope_heads(x, 2, cos, cos).shape == (B, 2, T, 64)
